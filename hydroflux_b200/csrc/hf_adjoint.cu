@@ -113,6 +113,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stage_adj(const StageArgs A, co
   const double inv_dx = 1.0 / dx, inv_dy = 1.0 / dy;
   const int tid = threadIdx.x;
   const int ntiles = A.tiles_x * A.tiles_y;
+  if (tid == 0) S.extreme = 0;
+  __syncthreads();
 
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int tyi = tile / A.tiles_x;
@@ -172,14 +174,14 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stage_adj(const StageArgs A, co
                        zfb);
         eta_cell = hc + S.z[c3];
         sex = S.sxe[isx(li, lj)];
-        eta_left = gj > 0 ? eta_cell - sex * (0.5 * dx) : eta_cell;
-        eta_right = gj + 1 < nc ? eta_cell + sex * (0.5 * dx) : eta_cell;
+        eta_left = gj > 0 ? eta_cell - sex : eta_cell;
+        eta_right = gj + 1 < nc ? eta_cell + sex : eta_cell;
         hfl = fmax(eta_left - zfl, 0.0);
         hfr = fmax(eta_right - zfr, 0.0);
         const double s_hu = hfa::div_rn((hfl + hfr) * ((eta_left - hfl) - (eta_right - hfr)) * (0.5 * GRAVITY), dx);
         sey = S.sye[isy(li, lj)];
-        eta_top = gi > 0 ? eta_cell - sey * (0.5 * dy) : eta_cell;
-        eta_bot = gi + 1 < nr ? eta_cell + sey * (0.5 * dy) : eta_cell;
+        eta_top = gi > 0 ? eta_cell - sey : eta_cell;
+        eta_bot = gi + 1 < nr ? eta_cell + sey : eta_cell;
         hft = fmax(eta_top - zft, 0.0);
         hfb = fmax(eta_bot - zfb, 0.0);
         const double s_hv = hfa::div_rn((hft + hfb) * ((eta_top - hft) - (eta_bot - hfb)) * (0.5 * GRAVITY), dy);
@@ -433,7 +435,6 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stage_adj(const StageArgs A, co
               const int m3 = i3(mi, mj), p3 = i3(pi, pj);
               const double zm = S.z[m3], zp = S.z[p3];
               const double zf = (dm != dp) ? fmax(zm, zp) : (zm + zp) * 0.5;
-              const double half = xd ? half_dx : half_dy;
               double se_m, sn_m, st_m, se_p, sn_p, st_p;
               if (xd) {
                 const int a = isx(mi, mj), b = isx(pi, pj);
@@ -444,12 +445,12 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stage_adj(const StageArgs A, co
                 se_m = S.sye[a]; sn_m = S.syv[a]; st_m = S.syu[a];
                 se_p = S.sye[b]; sn_p = S.syv[b]; st_p = S.syu[b];
               }
-              const double un_m = (xd ? S.u[m3] : S.v[m3]) + sn_m * half;
-              const double ut_m = (xd ? S.v[m3] : S.u[m3]) + st_m * half;
-              const double un_p = (xd ? S.u[p3] : S.v[p3]) - sn_p * half;
-              const double ut_p = (xd ? S.v[p3] : S.u[p3]) - st_p * half;
-              const double xm = (S.eta[m3] + se_m * half) - zf;
-              const double xp = (S.eta[p3] - se_p * half) - zf;
+              const double un_m = (xd ? S.u[m3] : S.v[m3]) + sn_m;
+              const double ut_m = (xd ? S.v[m3] : S.u[m3]) + st_m;
+              const double un_p = (xd ? S.u[p3] : S.v[p3]) - sn_p;
+              const double ut_p = (xd ? S.v[p3] : S.u[p3]) - st_p;
+              const double xm = (S.eta[m3] + se_m) - zf;
+              const double xp = (S.eta[p3] - se_p) - zf;
               const double h_m = fmax(xm, 0.0), h_p = fmax(xp, 0.0);
               double a0 = 0, a1 = 0, a2 = 0, b0 = 0, b1 = 0, b2 = 0;
               wb_face_rev(h_m, h_m * un_m, h_m * ut_m, h_p, h_p * un_p, h_p * ut_p, zf, lm, ln1,

@@ -167,6 +167,79 @@ __device__ __forceinline__ void wb_face(T hL, T qnL, T qtL, T hR, T qnR, T qtR, 
   tang = ft;
 }
 
+// The general face out of line, for the few faces of a moderate tile that
+// wb_face_wet leaves (kept out of the loop so that its registers do not
+// weigh on the common path).
+struct FaceFlux {
+  double mass, n_minus, n_plus, tang;
+};
+static __device__ __noinline__ FaceFlux wb_face_general(double hL, double qnL, double qtL, double hR,
+                                                 double qnR, double qtR, double zf) {
+  FaceFlux f;
+  wb_face<double>(hL, qnL, qtL, hR, qnR, qtR, zf, f.mass, f.n_minus, f.n_plus, f.tang);
+  return f;
+}
+
+// wb_face with both sides wet, for the faces of a tile whose inputs are all
+// moderate (hfa::moderate_or_zero; depths not negative). Same operations in
+// the same order, so the same values, with
+// - every quotient and root by the unguarded helpers (recip_rn, quo_*,
+//   sqrt_rn_moderate): six reciprocals serve the nine quotients;
+// - the sides' cases dropped: h > H_VEL on both sides makes the velocities
+//   plain quotients and every max(., 0) its argument, and hs > DRY_TOL makes
+//   both sides wet for HLLC, whose sampling is then three selects.
+// The divisors of the star state have known signs: denom < 0 (both products
+// subtract a speed from a bound on it), and s - s_star < 0 on the left and
+// > 0 on the right, where the numerator is >= +0, so quo_plus gives the IEEE
+// zeros. Returns false, with no flux, where a condition fails or a divisor's
+// low word is all ones; the caller then takes wb_face_general.
+//
+// Per face this is about 150 FP64 operations, the floor of a stage that is
+// bound by the FP64 pipe (two cycles per warp instruction and scheduler).
+__device__ __forceinline__ bool wb_face_wet(double hL, double unL_, double utL_, double hR,
+                                            double unR_, double utR_, double zf, FaceFlux& f) {
+  const double hsL = hL + zf - zf, hsR = hR + zf - zf;
+  if (!(hL > H_VEL && hR > H_VEL && hsL > DRY_TOL && hsR > DRY_TOL)) return false;
+  bool ones = hfa::low_word_ones(hL) || hfa::low_word_ones(hR) || hfa::low_word_ones(hsL) ||
+              hfa::low_word_ones(hsR);
+  double y = hfa::recip_rn(hL);
+  const double qnL = hsL * hfa::quo_keep(hL * unL_, hL, y);
+  const double qtL = hsL * hfa::quo_keep(hL * utL_, hL, y);
+  y = hfa::recip_rn(hR);
+  const double qnR = hsR * hfa::quo_keep(hR * unR_, hR, y);
+  const double qtR = hsR * hfa::quo_keep(hR * utR_, hR, y);
+  const double yL = hfa::recip_rn(hsL), yR = hfa::recip_rn(hsR);
+  const double unL = hfa::quo_keep(qnL, hsL, yL), unR = hfa::quo_keep(qnR, hsR, yR);
+  const double cl = hfa::sqrt_rn_moderate(hsL * GRAVITY);
+  const double cr = hfa::sqrt_rn_moderate(hsR * GRAVITY);
+  const double al = unL - cl, ar = unR - cr, bl = unL + cl, br = unR + cr;
+  const double sl = al < ar ? al : ar;
+  const double sr = bl > br ? bl : br;
+  const double tR = hsR * (unR - sr), tL = hsL * (unL - sl);
+  const double denom = tR - tL;
+  const double s_star = hfa::quo_plus(tR * sl - tL * sr, denom, hfa::recip_rn(denom));
+  const bool star = sl < 0.0 && sr > 0.0;
+  const bool left = star ? s_star >= 0.0 : sl >= 0.0;
+  const double h = left ? hsL : hsR, qn = left ? qnL : qnR, qt = left ? qtL : qtR;
+  const double un = left ? unL : unR, s = left ? sl : sr;
+  const double ut = hfa::quo_keep(qt, h, left ? yL : yR);
+  f.mass = qn;
+  double fn = qn * un + h * h * (0.5 * GRAVITY);
+  f.tang = qn * ut;
+  if (star) {
+    const double b = s - s_star;
+    ones = ones || hfa::low_word_ones(denom) || hfa::low_word_ones(b) ||
+           !(fabs(denom) > 1.0e-12);
+    const double hs = hfa::quo_plus(h * (s - un), b, hfa::recip_rn(b));
+    f.mass = qn + (hs - h) * s;
+    fn = fn + (hs * s_star - qn) * s;
+    f.tang = f.tang + (hs * ut - qt) * s;
+  }
+  f.n_minus = fn + (hL * hL - hsL * hsL) * (0.5 * GRAVITY);
+  f.n_plus = fn + (hR * hR - hsR * hsR) * (0.5 * GRAVITY);
+  return !ones;
+}
+
 // The reference's minmod(dl / d, dr / d) evaluated literally (update.rs:362-370).
 template <class T> __device__ __noinline__ T minmod_literal(T dl, T dr, double d) {
   const T a = dvp(dl, d), b = dvp(dr, d);  // d = dx or dy > 0
@@ -187,6 +260,54 @@ template <class T> __device__ __forceinline__ T minmod_div(T dl, T dr, const hfa
   if (!finite || fabs(l) < 1.0e-140 || fabs(r) < 1.0e-140) return minmod_literal<T>(dl, dr, rd.d);
   if (l * r <= 0.0) return cst<T>(0.0);
   return dvr(fabs(l) < fabs(r) ? dl : dr, rd);
+}
+
+// minmod_div for moderate operands and spacing (no quotient or product of
+// quotients under- or overflows): zero where the signs differ or an operand
+// is zero, else the quotient of the smaller magnitude. quo_plus makes every
+// zero +0, which is what the reference returns there.
+__device__ __forceinline__ double minmod_moderate(double l, double r, const hfa::RecipD& rd) {
+  double pick = fabs(l) < fabs(r) ? l : r;
+  if ((__double2hiint(l) ^ __double2hiint(r)) < 0) pick = 0.0;
+  return hfa::quo_plus(pick, rd.d, rd.hi);
+}
+
+// The stage's three operations with a guarded and a moderate (MOD, f64) form.
+// Limited slope of the middle one of three values.
+template <class T, bool MOD>
+__device__ __forceinline__ T limited_slope(T l, T c, T r, const hfa::RecipD& rd) {
+  if constexpr (MOD) return minmod_moderate(c - l, r - c, rd);
+  else return minmod_div<T>(c - l, r - c, rd);
+}
+// Face between two cells from their reconstructed depths (before the
+// max(., 0)) and velocities (update.rs:560-623).
+template <class T, bool MOD>
+__device__ __forceinline__ void face_interior(T hm, T un_m, T ut_m, T hp, T un_p, T ut_p, double zf,
+                                              T& m, T& n_minus, T& n_plus, T& tang) {
+  if constexpr (MOD) {
+    FaceFlux f;
+    if (!wb_face_wet(hm, un_m, ut_m, hp, un_p, ut_p, zf, f)) {
+      const double h_m = fmax(hm, 0.0), h_p = fmax(hp, 0.0);
+      f = wb_face_general(h_m, h_m * un_m, h_m * ut_m, h_p, h_p * un_p, h_p * ut_p, zf);
+    }
+    m = f.mass; n_minus = f.n_minus; n_plus = f.n_plus; tang = f.tang;
+  } else {
+    const T Z = cst<T>(0.0);
+    const T h_m = r_max(hm, Z), h_p = r_max(hp, Z);
+    wb_face<T>(h_m, h_m * un_m, h_m * ut_m, h_p, h_p * un_p, h_p * ut_p, zf, m, n_minus, n_plus,
+               tang);
+  }
+}
+// Face on a side of the grid, from a ghost's state.
+template <class T, bool MOD>
+__device__ __forceinline__ void face_side(T hL, T qnL, T qtL, T hR, T qnR, T qtR, double zf, T& m,
+                                          T& n_minus, T& n_plus, T& tang) {
+  if constexpr (MOD) {
+    const FaceFlux f = wb_face_general(hL, qnL, qtL, hR, qnR, qtR, zf);
+    m = f.mass; n_minus = f.n_minus; n_plus = f.n_plus; tang = f.tang;
+  } else {
+    wb_face<T>(hL, qnL, qtL, hR, qnR, qtR, zf, m, n_minus, n_plus, tang);
+  }
 }
 
 // Which operand minmod_div(dl, dr, d) returns: -1 for the constant zero, 0
@@ -213,6 +334,34 @@ __device__ __forceinline__ void friction_cell(T h, T& hu, T& hv, T n, double dt,
   const T factor = dv(n * n * speed, r_pow43(h)) * dt_g + 1.0;
   hu = dv(hu, factor);
   hv = dv(hv, factor);
+}
+
+// The same on f64 with the moderate helpers where the operands allow it:
+// h, n and dt within 2^+-60 and |q|^2 within 2^+-240 keep every
+// intermediate within 2^+-580 (the smaller momentum component is zero or at
+// least 2^-200). Water at rest (|q|^2 = 0) keeps its momentum: its factor is
+// 0 + 1.
+__device__ __forceinline__ void friction_moderate(double h, double& hu, double& hv, double n,
+                                                  double dt, double dry_tol) {
+  if (h <= dry_tol || n == 0.0) return;
+  const double dt_g = dt * GRAVITY;
+  const double q2 = hu * hu + hv * hv;
+  if (hfa::positive_within<60>(h) && hfa::positive_within<60>(n) &&
+      hfa::positive_within<60>(dt_g)) {
+    if (q2 == 0.0) return;
+    if (hfa::positive_within<240>(q2) && hfa::moderate_or_zero(hu) && hfa::moderate_or_zero(hv)) {
+      const double p = hfpow::pow_4_3(h);
+      const double speed = hfa::quo_keep(hfa::sqrt_rn_moderate(q2), h, hfa::recip_rn(h));
+      const double factor = hfa::quo_keep(n * n * speed, p, hfa::recip_rn(p)) * dt_g + 1.0;
+      if (!(hfa::low_word_ones(h) || hfa::low_word_ones(p) || hfa::low_word_ones(factor))) {
+        const double y = hfa::recip_rn(factor);
+        hu = hfa::quo_keep(hu, factor, y);
+        hv = hfa::quo_keep(hv, factor, y);
+        return;
+      }
+    }
+  }
+  friction_cell<double>(h, hu, hv, n, dt, dry_tol);
 }
 
 // Piecewise-linear series (same definition as the host forcing descriptor).
@@ -242,7 +391,22 @@ __device__ __forceinline__ double series_eval_u(const double* ts, const double* 
 // Wave speeds of an interior cell for the CFL bound (update.rs:121-135).
 __device__ __forceinline__ void cell_speeds(double h, double hu, double hv, double& sx,
                                             double& sy) {
-  if (!(h <= H_DRY)) {
+  if (h <= H_DRY) return;
+  if (hfa::positive_within<60>(h) && !hfa::low_word_ones(h) && hfa::moderate_or_zero(hu) &&
+      hfa::moderate_or_zero(hv)) {
+    const double c = hfa::sqrt_rn_moderate(GRAVITY * h);
+    double u = 0.0, v = 0.0;
+    if (h > H_VEL) {
+      const double y = hfa::recip_rn(h);
+      u = hfa::quo_keep(hu, h, y);
+      v = hfa::quo_keep(hv, h, y);
+    }
+    const double ax = fabs(u) + c, ay = fabs(v) + c;
+    sx = ax > sx ? ax : sx;
+    sy = ay > sy ? ay : sy;
+    return;
+  }
+  {
     // NaN depth: the reference's `h <= H_DRY` is false and sqrt(NaN) is
     // folded into f64::max, which ignores NaN; fmax does the same.
     const double c = sqrt(GRAVITY * h);

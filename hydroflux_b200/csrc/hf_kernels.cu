@@ -201,7 +201,7 @@ __global__ void k_friction(int64_t ncell, const double* __restrict__ n, double* 
        k += (int64_t)gridDim.x * blockDim.x) {
     double a = hu[k], b = hv[k];
     const double hh = h[k];
-    friction_cell(hh, a, b, n[k], dt, dry_tol);
+    friction_moderate(hh, a, b, n[k], dt, dry_tol);
     hu[k] = a;
     hv[k] = b;
   }

@@ -34,7 +34,10 @@ template <class T> struct StageSmemT {
   // eta, u and v start 8 bytes past a 16-byte boundary: the pipelined stage
   // stages z, hu and hv there with 16-byte copies of column pairs (even
   // global column, odd halo index), which then land on 16-byte boundaries.
-  double pad_;
+  // `extreme` fills the gap: set when a thread of the tile in hand meets a
+  // value that is not moderate, cleared before the next tile (and by the
+  // kernel before its first).
+  int extreme, pad_;
   T eta[R3N], u[R3N], v[R3N];
   T sxe[SXN], sxu[SXN], sxv[SXN];
   T sye[SYN], syu[SYN], syv[SYN];
@@ -45,7 +48,7 @@ template <class T> struct StageSmemT {
 using StageSmem = StageSmemT<double>;
 
 // The DualD tile would take 129 KB in the layout above: one CTA per SM. It
-// runs the x faces before the y faces (SplitFaces), so the y faces can be
+// runs the x faces before the y faces, so the y faces can be
 // written over the x momentum slopes (dead once the x faces are done) and
 // alpha over the y momentum slopes (dead once the y faces are done): 112 KB,
 // two CTAs per SM. The eta slopes of both directions stay (the bed source
@@ -65,8 +68,6 @@ template <> struct StageSmemT<DualD> {
     DualD a[AN];
   };
 };
-template <class T> struct SplitFaces { static constexpr bool value = false; };
-template <> struct SplitFaces<DualD> { static constexpr bool value = true; };
 
 __device__ __forceinline__ int i4(int li, int lj) { return (li + 4) * R4W + (lj + 4); }
 __device__ __forceinline__ int i3(int li, int lj) { return (li + 3) * R3W + (lj + 3); }
@@ -119,7 +120,10 @@ template <class T>
 __device__ __forceinline__ void finalize_cell(const StageArgs& A, const Ctrl* c, double dt,
                                               int gi, int gj, int64_t g, const int* order,
                                               int src_lo, int src_hi, T& h, T& hu, T& hv) {
-  friction_cell<T>(h, hu, hv, Field<T>::ld(A.n, A.tan.n, g), dt, A.dry_tol);
+  if constexpr (std::is_same<T, double>::value)
+    friction_moderate(h, hu, hv, A.n[g], dt, A.dry_tol);
+  else
+    friction_cell<T>(h, hu, hv, Field<T>::ld(A.n, A.tan.n, g), dt, A.dry_tol);
   if (c->rain_on) {
     const T nh = h + c->rain_dh;
     if (val(nh) <= 0.0) {
@@ -574,15 +578,28 @@ __device__ __forceinline__ void update_at(const StageArgs& A, SM& S, int gi0, in
 // DRY (forward stages of interior tiles only): when every depth of the tile
 // and its halo is at or below H_DRY, every cell of the tile takes the
 // isolated-dry update (update.rs:1072-1088), which reads no slope, face or
-// alpha: those phases are skipped and the function returns true. The vote
+// alpha: those phases are skipped and the function returns TILE_DRY. The vote
 // rides on the barrier that ends the primitives phase.
+// f64 tiles whose inputs are all moderate (hfa::moderate_or_zero, no negative
+// depth; checked while the primitives are formed) run their slopes and faces
+// with the unguarded division and square root and return TILE_MODERATE; the
+// others, which hold an extreme value, an infinity or a NaN, keep the
+// operation-by-operation tests. The values are the same.
+// The slope arrays hold slope * (spacing / 2), the only form in which the
+// faces and the bed source use a slope.
+enum TileClass { TILE_DRY, TILE_MODERATE, TILE_GENERAL };
+__device__ __forceinline__ bool moderate_cell(double h, double z, double hu, double hv) {
+  return __double2hiint(h) >= 0 && hfa::moderate_or_zero(h) && hfa::moderate_or_zero(z) &&
+         hfa::moderate_or_zero(hu) && hfa::moderate_or_zero(hv);
+}
 template <class T, bool PF = false, bool IN = false, bool DRY = false>
-__device__ __forceinline__ bool stage_tile_faces(const StageArgs& A, StageSmemT<T>& S, int gi0,
+__device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageSmemT<T>& S, int gi0,
                                                  int gj0, double dt, double* hst = nullptr,
                                                  int next = -1,
                                                  const StageArgs* next_args = nullptr) {
   constexpr bool SKIP = DRY && IN;
-  bool dry = true;
+  constexpr bool F64 = std::is_same<T, double>::value;
+  bool dry = true, mod = A.rx.moderate && A.ry.moderate;
   const int nr = A.nr, nc = A.nc;
   const double dx = A.dx, dy = A.dy;
   const double dt_dx = dt / dx;  // update.rs:930-931
@@ -601,18 +618,29 @@ __device__ __forceinline__ bool stage_tile_faces(const StageArgs& A, StageSmemT<
       if (r >= 1 && r < R4H - 1 && cc >= 1 && cc < R4W - 1) {
         const int k3 = (r - 1) * R3W + (cc - 1);
         const double zz = S.eta[k3], qu = S.u[k3], qv = S.v[k3];
+        const bool m = moderate_cell(hh, zz, qu, qv);
+        mod = mod && m;
         double uu = 0.0, vv = 0.0;
-        if (hh > H_VEL) dvp2(qu, qv, hh, uu, vv);
+        if (hh > H_VEL) {
+          if (m && !hfa::low_word_ones(hh)) {
+            const double y = hfa::recip_rn(hh);
+            uu = hfa::quo_keep(qu, hh, y);
+            vv = hfa::quo_keep(qv, hh, y);
+          } else {
+            dvp2(qu, qv, hh, uu, vv);
+          }
+        }
         S.z[k3] = zz;
         S.eta[k3] = hh + zz;
         S.u[k3] = uu;
         S.v[k3] = vv;
       }
     }
+    if (!mod) S.extreme = 1;
     if constexpr (SKIP) {
       if (__syncthreads_and(dry)) {
         if (next >= 0) stage_prefetch(next_args ? *next_args : A, S, hst, next);
-        return true;
+        return TILE_DRY;
       }
     } else {
       __syncthreads();
@@ -633,7 +661,20 @@ __device__ __forceinline__ bool stage_tile_faces(const StageArgs& A, StageSmemT<
         if (real) {
           zz = A.z[g];
           e = hh + zz;
-          if (val(hh) > H_VEL) {
+          if constexpr (F64) {
+            const double qu = A.in_hu[g], qv = A.in_hv[g];
+            const bool m = moderate_cell(hh, zz, qu, qv);
+            mod = mod && m;
+            if (hh > H_VEL) {
+              if (m && !hfa::low_word_ones(hh)) {
+                const double y = hfa::recip_rn(hh);
+                uu = hfa::quo_keep(qu, hh, y);
+                vv = hfa::quo_keep(qv, hh, y);
+              } else {
+                dvp2(qu, qv, hh, uu, vv);
+              }
+            }
+          } else if (val(hh) > H_VEL) {
             uu = dvp(Field<T>::ld(A.in_hu, A.tan.in_hu, g), hh);  // hh > H_VEL
             vv = dvp(Field<T>::ld(A.in_hv, A.tan.in_hv, g), hh);
           }
@@ -645,15 +686,21 @@ __device__ __forceinline__ bool stage_tile_faces(const StageArgs& A, StageSmemT<
       }
       if constexpr (SKIP) dry &= val(hh) <= H_DRY;
     }
+    if constexpr (F64) {
+      if (!mod) S.extreme = 1;
+    }
     if constexpr (SKIP) {
-      if (__syncthreads_and(dry)) return true;
+      if (__syncthreads_and(dry)) return TILE_DRY;
     } else {
       __syncthreads();
     }
   }
+  bool tile_mod = false;
+  if constexpr (F64) tile_mod = S.extreme == 0;
   {
     // ---- limited slopes: update.rs:459-540 (item k < SXN: x slope, else y)
-    auto slope_item = [&](int k) {
+    auto slope_item = [&](int k, auto mod_tag) {
+      constexpr bool MOD = decltype(mod_tag)::value;
       const bool xd = k < SXN;
       int li, lj;
       if (xd) {
@@ -692,10 +739,14 @@ __device__ __forceinline__ bool stage_tile_faces(const StageArgs& A, StageSmemT<
             sv = dvr(S.v[c3] - S.v[l3], rd);
           } else {
             const int l3 = c3 - st3, r3 = c3 + st3;
-            se = minmod_div<T>(S.eta[c3] - S.eta[l3], S.eta[r3] - S.eta[c3], rd);
-            su = minmod_div<T>(S.u[c3] - S.u[l3], S.u[r3] - S.u[c3], rd);
-            sv = minmod_div<T>(S.v[c3] - S.v[l3], S.v[r3] - S.v[c3], rd);
+            se = limited_slope<T, MOD>(S.eta[l3], S.eta[c3], S.eta[r3], rd);
+            su = limited_slope<T, MOD>(S.u[l3], S.u[c3], S.u[r3], rd);
+            sv = limited_slope<T, MOD>(S.v[l3], S.v[c3], S.v[r3], rd);
           }
+          const double half = xd ? half_dx : half_dy;
+          se = se * half;
+          su = su * half;
+          sv = sv * half;
         }
       }
       if (xd) {
@@ -710,7 +761,8 @@ __device__ __forceinline__ bool stage_tile_faces(const StageArgs& A, StageSmemT<
     };
 
     // ---- faces: update.rs:676-728 (face beds), 890-926 (fluxes) (item k < FXN: x face)
-    auto face_item = [&](int k) {
+    auto face_item = [&](int k, auto mod_tag) {
+      constexpr bool MOD = decltype(mod_tag)::value;
       const bool xd = k < FXN;
       int li, lj;  // x face: (row li, face lj); y face: (face li, column lj)
       if (xd) {
@@ -755,9 +807,9 @@ __device__ __forceinline__ bool stage_tile_faces(const StageArgs& A, StageSmemT<
         const T qn = xd ? hu : hv, qt = xd ? hv : hu;
         const T gqn = xd ? G.hu : G.hv, gqt = xd ? G.hv : G.hu;
         if (lo_side)
-          wb_face<T>(G.h, gqn, gqt, h, qn, qt, zf, m, nmn, npl, tg);
+          face_side<T, MOD>(G.h, gqn, gqt, h, qn, qt, zf, m, nmn, npl, tg);
         else
-          wb_face<T>(h, qn, qt, G.h, gqn, gqt, zf, m, nmn, npl, tg);
+          face_side<T, MOD>(h, qn, qt, G.h, gqn, gqt, zf, m, nmn, npl, tg);
       } else {
         const T hm = S.h[i4(mi, mj)], hp = S.h[i4(pi, pj)];
         const bool dm = val(hm) <= H_DRY, dp = val(hp) <= H_DRY;
@@ -767,7 +819,6 @@ __device__ __forceinline__ bool stage_tile_faces(const StageArgs& A, StageSmemT<
           const int m3 = i3(mi, mj), p3 = i3(pi, pj);
           const double zm = S.z[m3], zp = S.z[p3];
           const double zf = (dm != dp) ? fmax(zm, zp) : (zm + zp) * 0.5;  // update.rs:650-656
-          const double half = xd ? half_dx : half_dy;
           T se_m, sn_m, st_m, se_p, sn_p, st_p;
           if (xd) {
             const int a = isx(mi, mj), b = isx(pi, pj);
@@ -781,15 +832,13 @@ __device__ __forceinline__ bool stage_tile_faces(const StageArgs& A, StageSmemT<
           const T un_mc = xd ? S.u[m3] : S.v[m3], ut_mc = xd ? S.v[m3] : S.u[m3];
           const T un_pc = xd ? S.u[p3] : S.v[p3], ut_pc = xd ? S.v[p3] : S.u[p3];
           // reconstruct_x/y_face_states (update.rs:560-623)
-          const T eta_m = S.eta[m3] + se_m * half;
-          const T un_m = un_mc + sn_m * half;
-          const T ut_m = ut_mc + st_m * half;
-          const T eta_p = S.eta[p3] - se_p * half;
-          const T un_p = un_pc - sn_p * half;
-          const T ut_p = ut_pc - st_p * half;
-          const T h_m = r_max(eta_m - zf, Z);
-          const T h_p = r_max(eta_p - zf, Z);
-          wb_face<T>(h_m, h_m * un_m, h_m * ut_m, h_p, h_p * un_p, h_p * ut_p, zf, m, nmn, npl, tg);
+          const T eta_m = S.eta[m3] + se_m;
+          const T un_m = un_mc + sn_m;
+          const T ut_m = ut_mc + st_m;
+          const T eta_p = S.eta[p3] - se_p;
+          const T un_p = un_pc - sn_p;
+          const T ut_p = ut_pc - st_p;
+          face_interior<T, MOD>(eta_m - zf, un_m, ut_m, eta_p - zf, un_p, ut_p, zf, m, nmn, npl, tg);
         }
       }
       if (xd) {
@@ -800,17 +849,27 @@ __device__ __forceinline__ bool stage_tile_faces(const StageArgs& A, StageSmemT<
       }
     };
 
-    if constexpr (!SplitFaces<T>::value) {
-      for (int k = tid; k < SXN + SYN; k += NTHREADS) slope_item(k);
-      __syncthreads();
-      for (int k = tid; k < FXN + FYN; k += NTHREADS) face_item(k);
-      __syncthreads();
+    const std::true_type moderate{};
+    const std::false_type general{};
+    if constexpr (F64) {
+      if (tile_mod) {
+        for (int k = tid; k < SXN + SYN; k += NTHREADS) slope_item(k, moderate);
+        __syncthreads();
+        for (int k = tid; k < FXN + FYN; k += NTHREADS) face_item(k, moderate);
+        __syncthreads();
+      } else {
+        for (int k = tid; k < SXN + SYN; k += NTHREADS) slope_item(k, general);
+        __syncthreads();
+        if (tid == 0) S.extreme = 0;  // read by all before the barrier above
+        for (int k = tid; k < FXN + FYN; k += NTHREADS) face_item(k, general);
+        __syncthreads();
+      }
     } else {  // slopes, x faces, then y faces (over the x momentum slopes)
-      for (int k = tid; k < SXN + SYN; k += NTHREADS) slope_item(k);
+      for (int k = tid; k < SXN + SYN; k += NTHREADS) slope_item(k, general);
       __syncthreads();
-      for (int k = tid; k < FXN; k += NTHREADS) face_item(k);
+      for (int k = tid; k < FXN; k += NTHREADS) face_item(k, general);
       __syncthreads();
-      for (int k = FXN + tid; k < FXN + FYN; k += NTHREADS) face_item(k);
+      for (int k = FXN + tid; k < FXN + FYN; k += NTHREADS) face_item(k, general);
       __syncthreads();
     }
     if constexpr (PF) {
@@ -837,7 +896,7 @@ __device__ __forceinline__ bool stage_tile_faces(const StageArgs& A, StageSmemT<
     }
     __syncthreads();
   }
-  return false;
+  return tile_mod ? TILE_MODERATE : TILE_GENERAL;
 }
 
 // One forward-Euler stage (update.rs:805-1211) on one tile of one grid. Called
@@ -862,8 +921,15 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, StageSmemT<T>& S,
     const int tyi = tile / A.tiles_x;
     const int gi0 = tyi * TY, gj0 = (tile - tyi * A.tiles_x) * TX;
     // Dry interior tiles skip their slopes, faces and alpha (f64 forward stage).
-  stage_tile_faces<T, PF, IN, std::is_same<T, double>::value>(A, S, gi0, gj0, dt, hst, next,
-                                                                 next_args);
+    const bool mod = stage_tile_faces<T, PF, IN, std::is_same<T, double>::value>(
+                         A, S, gi0, gj0, dt, hst, next, next_args) == TILE_MODERATE;
+    // A source term's division by the spacing (moderate tiles: unguarded).
+    auto over = [mod](T a, const hfa::RecipD& r) -> T {
+      if constexpr (std::is_same<T, double>::value) {
+        if (mod) return hfa::quo_keep(a, r.d, r.hi);
+      }
+      return dvr(a, r);
+    };
 
     // ---- FV update + bed source + floor: update.rs:1071-1210
     int src_lo = 0, src_hi = 0;
@@ -916,17 +982,17 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, StageSmemT<T>& S,
         const double zc = S.z[c3];
         const T eta_cell = hc + zc;
         const T sex = S.sxe[isx(li, lj)];
-        const T eta_left = (IN || gj > 0) ? eta_cell - sex * (0.5 * dx) : eta_cell;
-        const T eta_right = (IN || gj + 1 < nc) ? eta_cell + sex * (0.5 * dx) : eta_cell;
+        const T eta_left = (IN || gj > 0) ? eta_cell - sex : eta_cell;
+        const T eta_right = (IN || gj + 1 < nc) ? eta_cell + sex : eta_cell;
         const T hfl = r_max(eta_left - zfl, Z);
         const T hfr = r_max(eta_right - zfr, Z);
-        const T s_hu = dvr((hfl + hfr) * ((eta_left - hfl) - (eta_right - hfr)) * (0.5 * GRAVITY), A.rx);
+        const T s_hu = over((hfl + hfr) * ((eta_left - hfl) - (eta_right - hfr)) * (0.5 * GRAVITY), A.rx);
         const T sey = S.sye[isy(li, lj)];
-        const T eta_top = (IN || gi > 0) ? eta_cell - sey * (0.5 * dy) : eta_cell;
-        const T eta_bot = (IN || gi + 1 < nr) ? eta_cell + sey * (0.5 * dy) : eta_cell;
+        const T eta_top = (IN || gi > 0) ? eta_cell - sey : eta_cell;
+        const T eta_bot = (IN || gi + 1 < nr) ? eta_cell + sey : eta_cell;
         const T hft = r_max(eta_top - zft, Z);
         const T hfb = r_max(eta_bot - zfb, Z);
-        const T s_hv = dvr((hft + hfb) * ((eta_top - hft) - (eta_bot - hfb)) * (0.5 * GRAVITY), A.ry);
+        const T s_hv = over((hft + hfb) * ((eta_top - hft) - (eta_bot - hfb)) * (0.5 * GRAVITY), A.ry);
 
         if (val(new_h) <= H_VEL) {
           nh = r_max(new_h, Z);  // moisture floor keeps the mass

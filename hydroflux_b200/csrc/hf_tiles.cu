@@ -119,6 +119,7 @@ __global__ void __launch_bounds__(NTHREADS, HF_MIN_BLOCKS) k_stage_pf(const Stag
   const int ntiles = A.tiles_x * A.tiles_y;
   double sxm = 0.0, sym = 0.0;
   unsigned long long nonfin = 0;
+  if (threadIdx.x == 0) P.s.extreme = 0;
   if ((int)blockIdx.x < ntiles) stage_prefetch(A, P.s, P.hst, blockIdx.x);
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     cp_async_wait_all();
@@ -263,6 +264,7 @@ __global__ void __launch_bounds__(NTHREADS, HF_MIN_BLOCKS)
   __shared__ int claimed;
   const int total_tiles = *n_tiles;  // device-resident: a graph serves any set of scenarios
   int t = blockIdx.x;
+  if (threadIdx.x == 0) P.s.extreme = 0;
   if (counter) {
     if (threadIdx.x == 0) claimed = atomicAdd(counter, 1);
     __syncthreads();
