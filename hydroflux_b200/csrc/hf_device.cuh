@@ -270,9 +270,10 @@ __device__ __forceinline__ bool wb_face_wet(double hL, double unL, double utL, d
 // faces, and 42% of the warps' passes over faces, come here (16 valleys of
 // sides 64 to 640, 72 steps: 47.7 -> 45.1 ms; a 1-step call at 700 x 500
 // 178.7 -> 171.7 us).
-static __device__ __noinline__ FaceFlux wb_face_moderate(double hm, double un_m, double ut_m,
-                                                         double hp, double un_p, double ut_p,
-                                                         double zf) {
+// Takes momenta; a negative depth's are not read.
+static __device__ __noinline__ FaceFlux wb_face_moderate_q(double hm, double qn_m, double qt_m,
+                                                           double hp, double qn_p, double qt_p,
+                                                           double zf) {
   FaceFlux f{0.0, 0.0, 0.0, 0.0};
   const double hL = __double2hiint(hm) < 0 ? 0.0 : hm, hR = __double2hiint(hp) < 0 ? 0.0 : hp;
   if (hL == 0.0 && hR == 0.0) return f;
@@ -288,13 +289,13 @@ static __device__ __noinline__ FaceFlux wb_face_moderate(double hm, double un_m,
     double qnR = 0.0, qtR = 0.0, unR = 0.0, utR = 0.0, cr = 0.0;
     if (hL > H_VEL) {
       const double y = hfa::recip_rn(hL);
-      qnL = hsL * hfa::quo_keep(hL * un_m, hL, y);
-      qtL = hsL * hfa::quo_keep(hL * ut_m, hL, y);
+      qnL = hsL * hfa::quo_keep(qn_m, hL, y);
+      qtL = hsL * hfa::quo_keep(qt_m, hL, y);
     }
     if (hR > H_VEL) {
       const double y = hfa::recip_rn(hR);
-      qnR = hsR * hfa::quo_keep(hR * un_p, hR, y);
-      qtR = hsR * hfa::quo_keep(hR * ut_p, hR, y);
+      qnR = hsR * hfa::quo_keep(qn_p, hR, y);
+      qtR = hsR * hfa::quo_keep(qt_p, hR, y);
     }
     if (wl) {
       const double y = hfa::recip_rn(hsL);
@@ -349,10 +350,16 @@ static __device__ __noinline__ FaceFlux wb_face_moderate(double hm, double un_m,
       f.tang = f.tang + (hs * ut - qt) * s;
     }
   }
-  if (ones) return wb_face_general(hL, hL * un_m, hL * ut_m, hR, hR * un_p, hR * ut_p, zf);
+  if (ones) return wb_face_general(hL, qn_m, qt_m, hR, qn_p, qt_p, zf);
   f.n_minus = fn + (hL * hL - hsL * hsL) * (0.5 * GRAVITY);
   f.n_plus = fn + (hR * hR - hsR * hsR) * (0.5 * GRAVITY);
   return f;
+}
+
+__device__ __forceinline__ FaceFlux wb_face_moderate(double hm, double un_m, double ut_m,
+                                                     double hp, double un_p, double ut_p,
+                                                     double zf) {
+  return wb_face_moderate_q(hm, hm * un_m, hm * ut_m, hp, hp * un_p, hp * ut_p, zf);
 }
 
 // The reference's minmod(dl / d, dr / d) evaluated literally (update.rs:362-370).
@@ -387,40 +394,28 @@ __device__ __forceinline__ double minmod_moderate(double l, double r, const hfa:
   return hfa::quo_plus(pick, rd.d, rd.hi);
 }
 
-// The stage's three operations with a guarded and a moderate (MOD, f64) form.
+// The stage's operations with a guarded and a moderate (MOD, f64) form.
 // Limited slope of the middle one of three values.
 template <class T, bool MOD>
 __device__ __forceinline__ T limited_slope(T l, T c, T r, const hfa::RecipD& rd) {
   if constexpr (MOD) return minmod_moderate(c - l, r - c, rd);
   else return minmod_div<T>(c - l, r - c, rd);
 }
+// Unlimited slope of a cell on a side from its one difference.
+template <class T, bool MOD>
+__device__ __forceinline__ T side_slope(T d, const hfa::RecipD& rd) {
+  if constexpr (MOD) return cst<T>(hfa::quo_keep(val(d), rd.d, rd.hi));
+  else return dvr(d, rd);
+}
 // Face between two cells from their reconstructed depths (before the
 // max(., 0)) and velocities (update.rs:560-623).
-template <class T, bool MOD>
+template <class T>
 __device__ __forceinline__ void face_interior(T hm, T un_m, T ut_m, T hp, T un_p, T ut_p, double zf,
                                               T& m, T& n_minus, T& n_plus, T& tang) {
-  if constexpr (MOD) {
-    FaceFlux f;
-    if (!wb_face_wet(hm, un_m, ut_m, hp, un_p, ut_p, zf, f))
-      f = wb_face_moderate(hm, un_m, ut_m, hp, un_p, ut_p, zf);
-    m = f.mass; n_minus = f.n_minus; n_plus = f.n_plus; tang = f.tang;
-  } else {
-    const T Z = cst<T>(0.0);
-    const T h_m = r_max(hm, Z), h_p = r_max(hp, Z);
-    wb_face<T>(h_m, h_m * un_m, h_m * ut_m, h_p, h_p * un_p, h_p * ut_p, zf, m, n_minus, n_plus,
-               tang);
-  }
-}
-// Face on a side of the grid, from a ghost's state.
-template <class T, bool MOD>
-__device__ __forceinline__ void face_side(T hL, T qnL, T qtL, T hR, T qnR, T qtR, double zf, T& m,
-                                          T& n_minus, T& n_plus, T& tang) {
-  if constexpr (MOD) {
-    const FaceFlux f = wb_face_general(hL, qnL, qtL, hR, qnR, qtR, zf);
-    m = f.mass; n_minus = f.n_minus; n_plus = f.n_plus; tang = f.tang;
-  } else {
-    wb_face<T>(hL, qnL, qtL, hR, qnR, qtR, zf, m, n_minus, n_plus, tang);
-  }
+  const T Z = cst<T>(0.0);
+  const T h_m = r_max(hm, Z), h_p = r_max(hp, Z);
+  wb_face<T>(h_m, h_m * un_m, h_m * ut_m, h_p, h_p * un_p, h_p * ut_p, zf, m, n_minus, n_plus,
+             tang);
 }
 
 // Which operand minmod_div(dl, dr, d) returns: -1 for the constant zero, 0
@@ -542,6 +537,20 @@ __device__ __forceinline__ void ghost_speeds(const Ghost& g, double& sx, double&
   const double v = hfa::div_rn(g.hv, h);
   sx = fmax(sx, fabs(u) + c);
   sy = fmax(sy, fabs(v) + c);
+}
+
+// The same for moderate ghosts; false, with nothing added, for others.
+__device__ __forceinline__ bool ghost_speeds_moderate(double h, double hu, double hv, double& sx,
+                                                      double& sy) {
+  if (h <= H_DRY) return true;
+  if (!(hfa::positive_within<60>(h) && !hfa::low_word_ones(h) && hfa::moderate_or_zero(hu) &&
+        hfa::moderate_or_zero(hv)))
+    return false;
+  const double c = hfa::sqrt_rn_moderate(GRAVITY * h), y = hfa::recip_rn(h);
+  const double ax = fabs(hfa::quo_keep(hu, h, y)) + c, ay = fabs(hfa::quo_keep(hv, h, y)) + c;
+  sx = ax > sx ? ax : sx;
+  sy = ay > sy ? ay : sy;
+  return true;
 }
 
 }  // namespace hf
