@@ -19,11 +19,14 @@ OUT = os.path.join(HERE, "libhydroflux_gpu.so")
 
 SOURCES = ["hf_kernels.cu", "hf_tiles.cu", "hf_api.cu", "hf_noalloc.cu", "hf_batch.cu",
            "hf_serve.cu", "hf_adjoint.cu", "hf_calib.cu", "hf_io.cu"]
-# hf_tiles.cu is compiled once more for the 32 x 32 tile geometry (the
-# default macros give the 32 x 8 one; see hf_internal.h).
-GEOM_LARGE = ("hf_tiles.cu", "hf_tiles_g32.o",
-              ["-DHF_GEOM=g32", "-DHF_GEOM_INDEX=1", "-DHF_TILE_Y=32", "-DHF_THREADS=1024",
-               "-DHF_MIN_BLOCKS=1"])
+# hf_tiles.cu is compiled once more for each other tile geometry (the default
+# macros give 32 x 8 tiles by 256 threads; see hf_internal.h).
+GEOMETRIES = [("hf_tiles.cu", "hf_tiles_%s.o" % name,
+               ["-DHF_GEOM=" + name, "-DHF_GEOM_INDEX=%d" % index, "-DHF_TILE_Y=%d" % rows,
+                "-DHF_THREADS=%d" % threads, "-DHF_MIN_BLOCKS=%d" % blocks])
+              for name, index, rows, threads, blocks in (
+                  ("g32", 1, 32, 1024, 1), ("g8w", 2, 8, 768, 1), ("g8m", 3, 8, 384, 2),
+                  ("g4", 4, 4, 512, 1))]
 GENCODE = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--fmad=false", "-prec-div=true",
               "-prec-sqrt=true", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",
@@ -56,7 +59,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
         return OUT
     objdir = os.path.join(HERE, "_build")
     os.makedirs(objdir, exist_ok=True)
-    units = [(src, src.replace(".cu", ".o"), []) for src in SOURCES] + [GEOM_LARGE]
+    units = [(src, src.replace(".cu", ".o"), []) for src in SOURCES] + GEOMETRIES
     objs, procs = [], []
     for src, name, defs in units:  # the translation units compile in parallel
         obj = os.path.join(objdir, name)

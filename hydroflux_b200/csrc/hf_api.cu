@@ -241,8 +241,9 @@ ForcingDev ForcingHost::dev(int geom) const {
   f.src_off = d_off;
   f.src_t = d_st;
   f.src_q = d_sq;
-  f.tile_start = d_tile_start[geom];
-  f.tile_order = d_tile_order[geom];
+  const int b = geom == kGeomLarge ? 1 : 0;
+  f.tile_start = d_tile_start[b];
+  f.tile_order = d_tile_order[b];
   f.blk_start = d_blk_start;
   f.blk_order = d_blk_order;
   f.src_dh = d_dh;
@@ -290,7 +291,7 @@ int hf::forcing_set_sources(ForcingHost& f, int64_t nr, int64_t nc, int64_t n_so
     c[k] = (int)cols[k];
   }
   for (int k = 0; k <= ns; ++k) off[k] = (int)offsets[k];
-  // Bucket the sources by the stage tiles of each geometry and by strip
+  // Bucket the sources by the stage tiles of 8 and of 32 rows and by strip
   // block, keeping their order within a bucket (repeated cells accumulate in
   // the caller's order).
   auto bucket = [&](int nbuckets, auto key, std::vector<int>& start, std::vector<int>& order) {
@@ -358,8 +359,7 @@ struct hf_sim {
   ForcingHost forcing;
   GaugeDev gauge{};  // n == 0: no gauges
   cudaGraphExec_t graphs[3] = {nullptr, nullptr, nullptr};
-  // Tile geometry of the tile-shaped kernels (kGeomSmall / kGeomLarge) and
-  // its entry points; tiles_x, tiles_y and grid are in its tiles.
+  // Tile geometry of the tile-shaped kernels (kGeom*) and its entry points; tiles_x, tiles_y and grid are in its tiles.
   int geom = kGeomSmall;
   const GeomOps* ops = nullptr;
   // Stage kernel: HF_STAGE_TILE / HF_STAGE_TILE32 (k_stage_pf of the 32 x 8
@@ -433,16 +433,20 @@ void set_geom(hf_sim* s, int geom) {
 
 // Picks the stage kernel: the strip kernel where it is asked for and its TMA
 // descriptors can be made, else the tile kernel of the geometry asked for;
-// auto takes the tile kernel of the grid's geometry (geom_for: on B200 the
+// auto takes the tile kernel of the grid's geometry (geom_pick: on B200 the
 // tile kernel measured faster than the strip kernel on wet grids and as fast
 // on mostly dry ones). The strip kernel's grids keep the 32 x 8 geometry for
 // the CFL reduction and the forward-Euler finalize.
 int choose_stage_kernel(hf_sim* s, int kind) {
-  const int geom = kind == HF_STAGE_TILE32   ? kGeomLarge
-                   : kind == HF_STAGE_AUTO ? geom_for(s->nr, s->nc)
-                                           : kGeomSmall;
+  const int64_t tx = tiles_along(s->nc, TX);
+  const int geom = kind == HF_STAGE_TILE32 ? kGeomLarge
+                   : kind == HF_STAGE_AUTO ? geom_pick(s->nr, s->nc)
+                   : kind == HF_STAGE_TILE
+                       ? small_geom(tx * tiles_along(s->nr, 8), tx * tiles_along(s->nr, 4))
+                       : kGeomSmall;
   set_geom(s, geom);
-  s->stage_kind = geom == kGeomLarge ? HF_STAGE_TILE32 : HF_STAGE_TILE;
+  const int as = kind == HF_STAGE_AUTO ? geom_for(s->nr, s->nc) : geom;
+  s->stage_kind = as == kGeomLarge ? HF_STAGE_TILE32 : HF_STAGE_TILE;
   if (kind != HF_STAGE_STRIP) return HF_OK;
   int g = strip_grid_size(s->nr, s->nc, s->device);
   if (g == 0) {  // a small grid: one CTA per block at most
@@ -653,7 +657,7 @@ int hf_sim_create(const hf_mesh_desc* mesh, const double* h, const double* hu, c
   s->dx = mesh->dx;
   s->dy = mesh->dy;
   s->cfg = *cfg;
-  set_geom(s, geom_for(s->nr, s->nc));
+  set_geom(s, geom_pick(s->nr, s->nc));
   int rc = HF_OK;
   auto done = [&](int code) {
     if (code != HF_OK) destroy_sim(s);
@@ -1181,7 +1185,7 @@ int euler_like(const hf_grid* grid, double* h, double* hu, double* hv, const hf_
   const hf_boundaries b = bcs ? *bcs : transmissive();
   HF_TRY(check_bcs(b, grid->n_rows, grid->n_cols));
   DeviceGuard guard(w->device);
-  const GeomOps& o = geom_ops(geom_for(grid->n_rows, grid->n_cols));
+  const GeomOps& o = geom_ops(geom_pick(grid->n_rows, grid->n_cols));
   StageArgs a = ws_args(grid, b, w, o);
   const int gsz = o.grid_size(a.tiles_x * a.tiles_y, w->device);
   HF_TRY(launch_set_fixed(w->d_ctrl, dt, stream));
@@ -1217,7 +1221,7 @@ int hf_cfl_time_step(const hf_grid* grid, const double* h, const double* hu, con
   }
   DeviceGuard guard(w->device);
   cudaStream_t st = (cudaStream_t)stream;
-  const GeomOps& o = geom_ops(geom_for(grid->n_rows, grid->n_cols));
+  const GeomOps& o = geom_ops(geom_pick(grid->n_rows, grid->n_cols));
   StageArgs a = ws_args(grid, bcs ? *bcs : transmissive(), w, o);
   a.in_h = h; a.in_hu = hu; a.in_hv = hv;
   HF_CUDA(cudaMemsetAsync(&w->d_ctrl->sx_bits, 0, 3 * sizeof(unsigned long long), st));

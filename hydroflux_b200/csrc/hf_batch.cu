@@ -72,8 +72,8 @@ constexpr int kSchedules = 4;  // bit 0: dynamic; bit 1: largest scenarios first
 struct hf_batch {
   int device = 0;
   cudaStream_t stream = nullptr;
-  // Tile geometry of the batched kernels: 32 x 32 once the batched scenarios
-  // have kLargeTilesMin such tiles between them, else 32 x 8.
+  // Tile geometry of the batched kernels, picked by the tiles of all batched
+  // scenarios as a single grid's is (small_tiles_pay, small_geom).
   int geom = kGeomSmall;
   const GeomOps* ops = nullptr;
   // Scenarios of at least kSoloTilesMin tiles of 32 x 32 are not in the tile
@@ -284,8 +284,6 @@ int hf_batch_create(int64_t n_scenarios, const hf_scenario_desc* sc, int device,
     tiles += tx * tiles_along(d.mesh.n_rows, kGeomTileH[kGeomSmall]);
     tiles_large += t32;
   }
-  const int geom = tiles_large >= kLargeTilesMin ? kGeomLarge : kGeomSmall;
-  if (geom == kGeomLarge) tiles = tiles_large;
   if (tiles > INT_MAX / 2) return bfail(HF_ERR_INVALID_ARG, "ensemble too large");
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || device < 0 || device >= ndev) {
@@ -293,6 +291,8 @@ int hf_batch_create(int64_t n_scenarios, const hf_scenario_desc* sc, int device,
     return bfail(HF_ERR_CUDA, "no such CUDA device");
   }
   Guard guard(device);
+  const int geom = small_tiles_pay(tiles, tiles_large) ? small_geom(tiles, 0) : kGeomLarge;
+  if (geom == kGeomLarge) tiles = tiles_large;
   hf_batch* b = new hf_batch();
   auto done = [&](int code) {
     if (code != HF_OK) destroy_batch(b);

@@ -14,8 +14,9 @@ namespace hf {
 // Tile geometry of the fused stage kernels: a CTA advances a TX x TY block
 // of cells, one cell per thread; its shared-memory halo is 4 cells (two-cell
 // dry buffer of the slope limiter + one neighbour slope + one neighbour
-// alpha). Two geometries are built (hf_tiles.cu is compiled once for each;
-// its symbols sit in the geometry's inline namespace):
+// alpha). hf_tiles.cu is compiled once for each geometry, whose symbols sit in
+// its inline namespace; geom_pick() says which one a grid takes. Two carry the
+// grids that fill the GPU:
 // - 32 x 8 (g8, kGeomSmall): 256 threads, 71 KB of shared memory, three CTAs
 //   (24 warps) per SM. Many tiles per grid, so small grids still spread over
 //   every SM. The DualD tangent, the adjoint, the strip kernel and the
@@ -24,15 +25,20 @@ namespace hf {
 //   CTA (32 warps) per SM. The halo is a smaller share of the tile (2.32
 //   Audusse+HLLC faces and 2.39 limited-slope cells per cell against 2.83
 //   and 3.0) and an SM runs more warps; a stage launch on the 4096^2 valley
-//   takes 2.06 ms against 2.36 ms. Grids with at least kLargeTilesMin tiles
-//   of it take it (geom_for).
-// Both compute every cell with the same operations: results are identical.
+//   takes 1.60 ms against 1.79 ms.
+// Grids that leave SMs idle are bound by the latency of one tile: its five
+// phases take about three passes of 256 threads each. They run on CTAs with
+// more threads per tile (us a step, wet with walls, 256 threads -> the other):
+// - 32 x 8, 768 threads (g8w, kGeomWide): one pass per phase, one CTA per SM;
+//   160 x 200 31.1 -> 26.2, but 256^2 (two tiles for some SMs) 35.3 -> 39.0.
+// - 32 x 8, 384 threads (g8m, kGeomMid): two passes, two CTAs per SM; 256^2
+//   35.3 -> 32.1, but 199 x 481 (400 tiles) 39.8 -> 44.7.
+// - 32 x 4, 512 threads (g4, kGeomLow): half the work per SM again; 48 x 64
+//   24.9 (g8w) -> 22.8.
+// All compute every cell with the same operations: results are identical.
 constexpr int TX = 32;
-constexpr int kGeomSmall = 0, kGeomLarge = 1;
-#ifndef HF_LARGE_TILE_Y
-#define HF_LARGE_TILE_Y 32  // the large geometry's tile height (build.py passes the same)
-#endif
-constexpr int kGeomTileH[2] = {8, HF_LARGE_TILE_Y};
+constexpr int kGeomSmall = 0, kGeomLarge = 1, kGeomWide = 2, kGeomMid = 3, kGeomLow = 4;
+constexpr int kGeomTileH[5] = {8, 32, 8, 8, 4};
 constexpr int kLargeTilesMin = 100;
 // A scenario of an ensemble or server with at least this many 32 x 32 tiles
 // (about 3.5 waves of the 148 SMs; from 724 x 724 cells on) fills the GPU
@@ -63,6 +69,12 @@ constexpr int CELLS_PER_THREAD = (TY + ROWS_PER_PASS - 1) / ROWS_PER_PASS;
 constexpr bool kPartialPass = TY % ROWS_PER_PASS != 0;
 static_assert(NTHREADS % TX == 0, "tile / thread shape");
 static_assert(TY == kGeomTileH[HF_GEOM_INDEX], "geometry index and tile height");
+// Point sources are bucketed by tiles of 8 or 32 rows (ForcingHost); lower
+// tiles look into the bucket around them.
+constexpr int kBucketRows = TY < 8 ? 8 : TY;
+HF_ARITH_HD int source_bucket(int tile, int tiles_x) {
+  return TY == kBucketRows ? tile : tile / tiles_x / (kBucketRows / TY) * tiles_x + tile % tiles_x;
+}
 }  // namespace HF_GEOM
 
 // Strip geometry of the streaming stage kernel (hf_strip.cuh): a CTA walks
@@ -275,10 +287,24 @@ struct GeomOps {
 };
 const GeomOps& geom_ops_g8();
 const GeomOps& geom_ops_g32();
+const GeomOps& geom_ops_g8w();
+const GeomOps& geom_ops_g8m();
+const GeomOps& geom_ops_g4();
 const GeomOps& geom_ops(int geom);
-// The geometry of an nr x nc grid: kGeomLarge once it has kLargeTilesMin
-// tiles of 32 x 32, else kGeomSmall.
+// The stage kernel kind a simulation reports for an nr x nc grid: kGeomLarge
+// once it has kLargeTilesMin tiles of 32 x 32, else kGeomSmall.
 int geom_for(int64_t nr, int64_t nc);
+// The geometry that runs it on the current device. Tiles of 32 x 8 or 32 x 32
+// by the time of their waves (3 and 1 tiles per SM; a wave of a step takes
+// about 19 to 24 and 28.5 us; us a step with small and large tiles, wet:
+// 199 x 481 39.0 / 45.2, 400^2 60 / 74, 450 x 500 80 / 75, 512^2 78 / 77,
+// 700 x 500 95 / 102, 1024^2 242 / 214), and among the small ones
+// (small_geom) the CTA that fills the SMs.
+int geom_pick(int64_t nr, int64_t nc);
+// Whether n8 tiles of 32 x 8 take less time than n32 of 32 x 32 on the device.
+bool small_tiles_pay(int64_t n8, int64_t n32);
+// The small geometry of n8 tiles of 32 x 8 (n4 of 32 x 4; 0: not asked for).
+int small_geom(int64_t n8, int64_t n4);
 inline int tiles_along(int64_t n, int tile) { return (int)((n + tile - 1) / tile); }
 
 inline namespace HF_GEOM {
@@ -383,7 +409,7 @@ struct ForcingHost {
   int* d_off = nullptr;
   double* d_st = nullptr;
   double* d_sq = nullptr;
-  int* d_tile_start[2] = {nullptr, nullptr};  // per geometry (kGeomSmall, kGeomLarge)
+  int* d_tile_start[2] = {nullptr, nullptr};  // tiles of 8 and of 32 rows
   int* d_tile_order[2] = {nullptr, nullptr};
   int* d_blk_start = nullptr;
   int* d_blk_order = nullptr;

@@ -331,11 +331,47 @@ int elem_grid(int64_t n) {
 
 cudaError_t last_launch_error() { return g_launch_error; }
 
-const GeomOps& geom_ops(int geom) { return geom == kGeomLarge ? geom_ops_g32() : geom_ops_g8(); }
+const GeomOps& geom_ops(int geom) {
+  switch (geom) {
+    case kGeomLarge: return geom_ops_g32();
+    case kGeomWide: return geom_ops_g8w();
+    case kGeomMid: return geom_ops_g8m();
+    case kGeomLow: return geom_ops_g4();
+    default: return geom_ops_g8();
+  }
+}
 
 int geom_for(int64_t nr, int64_t nc) {
   const int64_t t = (int64_t)tiles_along(nc, TX) * tiles_along(nr, kGeomTileH[kGeomLarge]);
   return t >= kLargeTilesMin ? kGeomLarge : kGeomSmall;
+}
+
+namespace {
+int64_t sm_count() {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    cudaGetLastError();
+  return sms > 0 ? sms : 148;
+}
+}  // namespace
+
+bool small_tiles_pay(int64_t n8, int64_t n32) {
+  const int64_t sms = sm_count(), w8 = (n8 + 3 * sms - 1) / (3 * sms);
+  // tenths of a microsecond; from five waves on CTAs drift apart and only the
+  // number of tiles counts
+  const int64_t t8 = w8 <= 4 ? 190 * w8 + 40 : 243 * n8 / (3 * sms);
+  return t8 < 285 * ((n32 + sms - 1) / sms);
+}
+int small_geom(int64_t n8, int64_t n4) {
+  const int64_t sms = sm_count();
+  if (n4 > 0 && n4 <= sms) return kGeomLow;
+  return n8 <= sms ? kGeomWide : n8 <= 2 * sms ? kGeomMid : kGeomSmall;
+}
+int geom_pick(int64_t nr, int64_t nc) {
+  const int64_t tx = tiles_along(nc, TX), n8 = tx * tiles_along(nr, 8);
+  return small_tiles_pay(n8, tx * tiles_along(nr, 32)) ? small_geom(n8, tx * tiles_along(nr, 4))
+                                                       : kGeomLarge;
 }
 
 namespace {

@@ -130,7 +130,7 @@ extern "C" int hf_ssprk2_step_noalloc(const hf_grid* grid, double* h, double* hu
     cudaGetLastError();
     return noalloc_fail(HF_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
   }
-  const GeomOps& o = geom_ops(geom_for(grid->n_rows, grid->n_cols));
+  const GeomOps& o = geom_ops(geom_pick(grid->n_rows, grid->n_cols));
   StageArgs a;
   std::memset(&a, 0, sizeof a);
   a.nr = (int)grid->n_rows;

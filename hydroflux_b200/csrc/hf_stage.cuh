@@ -968,8 +968,9 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, StageSmemT<T>& S,
     // ---- FV update + bed source + floor: update.rs:1071-1210
     int src_lo = 0, src_hi = 0;
     if (A.finalize && A.f.n_src > 0) {
-      src_lo = A.f.tile_start[tile];
-      src_hi = A.f.tile_start[tile + 1];
+      const int b = source_bucket(tile, A.tiles_x);
+      src_lo = A.f.tile_start[b];
+      src_hi = A.f.tile_start[b + 1];
     }
 #pragma unroll 1
     for (int q = 0; q < CELLS_PER_THREAD; ++q) {

@@ -332,8 +332,9 @@ __device__ void finalize_tiles(const StageArgs& A, Ctrl* ctrl, double& sxm, doub
     const int gi0 = tyi * TY, gj0 = (tile - tyi * A.tiles_x) * TX;
     int src_lo = 0, src_hi = 0;
     if (A.f.n_src > 0) {
-      src_lo = A.f.tile_start[tile];
-      src_hi = A.f.tile_start[tile + 1];
+      const int b = source_bucket(tile, A.tiles_x);
+      src_lo = A.f.tile_start[b];
+      src_hi = A.f.tile_start[b + 1];
     }
     for (int q = 0; q < CELLS_PER_THREAD; ++q) {
       if (kPartialPass && (int)threadIdx.x / TX + ROWS_PER_PASS * q >= TY) continue;
