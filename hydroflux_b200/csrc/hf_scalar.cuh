@@ -108,11 +108,18 @@ __device__ __forceinline__ DualD r_sqrt_pos(DualD x) { return r_sqrt(x); }
 // max / min (dual.rs:130-155): ties average the derivatives.
 __device__ __forceinline__ double r_max(double a, double b) { return fmax(a, b); }
 __device__ __forceinline__ double r_min(double a, double b) { return fmin(a, b); }
+// max(x, 0) of the result of an operation (a NaN there has its quiet bit, so
+// its high word is above infinity's): a test of the high word instead of the
+// compares and selects of fmax.
+__device__ __forceinline__ double r_max0(double x) {
+  return (unsigned)__double2hiint(x) <= 0x7ff00000u ? x : 0.0;
+}
 __device__ __forceinline__ DualD r_max(DualD a, DualD b) {
   if (a.v > b.v) return a;
   if (b.v > a.v) return b;
   return DualD{a.v, 0.5 * (a.d + b.d)};
 }
+__device__ __forceinline__ DualD r_max0(DualD x) { return r_max(x, DualD{0.0, 0.0}); }
 __device__ __forceinline__ DualD r_min(DualD a, DualD b) {
   if (a.v < b.v) return a;
   if (b.v < a.v) return b;

@@ -28,6 +28,17 @@ constexpr int FXW = TX + 3, FXH = TY + 2, FXN = FXW * FXH;  // x faces: rows [-1
 constexpr int FYW = TX + 2, FYH = TY + 3, FYN = FYW * FYH;  // y faces: faces [-1,TY+1], cols [-1,TX]
 constexpr int AW = TX + 2, AH = TY + 2, AN = AW * AH;       // alpha: rows [-1,TY], cols [-1,TX]
 
+// The dry cells (h <= H_DRY, inside the grid) of a row of the tile and its
+// halo: bit c is column c - 4. The limiter, the faces and the update test
+// dryness about 22 times per cell; a test of bits takes none of the FP64 pipe
+// and one load for the neighbours of a row.
+struct alignas(8) DryRow {
+  unsigned lo, hi;
+};
+__device__ __forceinline__ unsigned dry_window(const DryRow& d, int lj) {  // bit k: column lj + k
+  return (unsigned)((((unsigned long long)d.hi << 32) | d.lo) >> (lj + 4));
+}
+
 template <class T> struct StageSmemT {
   T h[R4N];
   double z[R3N];
@@ -44,6 +55,7 @@ template <class T> struct StageSmemT {
   T fxm[FXN], fxnm[FXN], fxnp[FXN], fxt[FXN];  // mass, normal(minus), normal(plus), tangential
   T fym[FYN], fynm[FYN], fynp[FYN], fyt[FYN];
   T a[AN];
+  DryRow dry[R4H];
 };
 using StageSmem = StageSmemT<double>;
 
@@ -67,7 +79,24 @@ template <> struct StageSmemT<DualD> {
     struct { DualD syu[SYN], syv[SYN]; };
     DualD a[AN];
   };
+  DryRow dry[R4H];
 };
+
+// The cells of the tile with its 4-cell halo by warps: rows of 32 columns,
+// then the last 8 columns of four rows at a time.
+constexpr int HALO_WARPS = R4H + R4H / 4;
+static_assert(R4W == 40 && R4H % 4 == 0, "halo items");
+__device__ __forceinline__ void halo_item(int w, int lane, int& r, int& cc) {
+  r = w < R4H ? w : (w - R4H) * 4 + (lane >> 3);
+  cc = w < R4H ? lane : 32 + (lane & 7);
+}
+__device__ __forceinline__ void dry_store(DryRow* dry, int w, int lane, int r, unsigned ballot) {
+  if (w < R4H) {
+    if (lane == 0) dry[r].lo = ballot;
+  } else if ((lane & 7) == 0) {
+    dry[r].hi = (ballot >> lane) & 0xffu;
+  }
+}
 
 __device__ __forceinline__ int i4(int li, int lj) { return (li + 4) * R4W + (lj + 4); }
 __device__ __forceinline__ int i3(int li, int lj) { return (li + 3) * R3W + (lj + 3); }
@@ -622,11 +651,16 @@ __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageS
   if constexpr (PF) {
     // ---- depth snapshot and primitives from the staged inputs. Cells outside
     // the grid were zero-filled, so they get h = z = eta = u = v = +0 as below.
-    for (int k = tid; k < R4N; k += NTHREADS) {
-      const int r = k / R4W, cc = k - r * R4W;
+    for (int w = tid >> 5; w < HALO_WARPS; w += NTHREADS / 32) {
+      int r, cc;
+      halo_item(w, tid & 31, r, cc);
+      const int k = r * R4W + cc;
       const double hh = hst[k];
+      const bool real = IN || (gi0 + r >= 4 && gi0 + r < nr + 4 && gj0 + cc >= 4 && gj0 + cc < nc + 4);
+      const bool d = hh <= H_DRY;
+      dry_store(S.dry, w, tid & 31, r, __ballot_sync(0xffffffffu, real && d));
       S.h[k] = hh;
-      if constexpr (SKIP) dry &= hh <= H_DRY;
+      if constexpr (SKIP) dry &= d;
       if (r >= 1 && r < R4H - 1 && cc >= 1 && cc < R4W - 1) {
         const int k3 = (r - 1) * R3W + (cc - 1);
         const double zz = S.eta[k3], qu = S.u[k3], qv = S.v[k3];
@@ -659,12 +693,15 @@ __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageS
     }
   } else {
     // ---- depth snapshot (halo 4) and primitives (halo 3): update.rs:853-858, 405-426
-    for (int k = tid; k < R4N; k += NTHREADS) {
-      const int r = k / R4W, cc = k - r * R4W;
+    for (int w = tid >> 5; w < HALO_WARPS; w += NTHREADS / 32) {
+      int r, cc;
+      halo_item(w, tid & 31, r, cc);
+      const int k = r * R4W + cc;
       const int gi = gi0 + r - 4, gj = gj0 + cc - 4;
       const bool real = IN || (gi >= 0 && gi < nr && gj >= 0 && gj < nc);
       const int64_t g = (int64_t)gi * nc + gj;
       const T hh = real ? Field<T>::ld(A.in_h, A.tan.in_h, g) : Z;
+      dry_store(S.dry, w, tid & 31, r, __ballot_sync(0xffffffffu, real && val(hh) <= H_DRY));
       S.h[k] = hh;
       if (r >= 1 && r < R4H - 1 && cc >= 1 && cc < R4W - 1) {
         const int k3 = (r - 1) * R3W + (cc - 1);
@@ -728,15 +765,19 @@ __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageS
       if (!IN && (gi < 0 || gi >= nr || gj < 0 || gj >= nc)) return;
       const int ga = xd ? gj : gi;
       const int na = xd ? nc : nr;
-      const int st4 = xd ? 1 : R4W;
       const int st3 = xd ? 1 : R3W;
       const hfa::RecipD& rd = xd ? A.rx : A.ry;
       T se = Z, su = Z, sv = Z;
       if (IN || na >= 2) {
-        const int lo = IN ? -2 : max(ga - 2, 0) - ga, hi = IN ? 2 : min(ga + 2, na - 1) - ga;
-        const int c4 = i4(li, lj);
-        bool anyd = false;
-        for (int o = lo; o <= hi; ++o) anyd |= val(S.h[c4 + o * st4]) <= H_DRY;
+        bool anyd;
+        if (xd) {
+          anyd = (dry_window(S.dry[li + 4], lj - 2) & 31u) != 0;
+        } else {
+          const DryRow* d = &S.dry[li + 2];
+          const DryRow any{d[0].lo | d[1].lo | d[2].lo | d[3].lo | d[4].lo,
+                           d[0].hi | d[1].hi | d[2].hi | d[3].hi | d[4].hi};
+          anyd = (dry_window(any, lj) & 1u) != 0;
+        }
         if (!anyd) {
           const int c3 = i3(li, lj);
           if (!IN && (ga == 0 || ga == na - 1)) {  // one-sided: / dx or / dy
@@ -830,7 +871,15 @@ __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageS
           wb_face<T>(hm, qnm, qtm, hp, qnp, qtp, zf, m, nmn, npl, tg);
         }
       } else {
-        const bool dm = val(S.h[i4(mi, mj)]) <= H_DRY, dp = val(S.h[i4(pi, pj)]) <= H_DRY;
+        bool dm, dp;
+        if (xd) {
+          const unsigned d = dry_window(S.dry[pi + 4], mj);
+          dm = d & 1u;
+          dp = d & 2u;
+        } else {
+          dm = dry_window(S.dry[mi + 4], pj) & 1u;
+          dp = dry_window(S.dry[pi + 4], pj) & 1u;
+        }
         if (!(dm && dp)) {
           const int m3 = i3(mi, mj), p3 = i3(pi, pj);
           const double zm = S.z[m3], zp = S.z[p3];
@@ -925,7 +974,7 @@ __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageS
       if (val(fl) < 0.0) out = out + (-fl) * dt_dx;
       if (val(fb) > 0.0) out = out + fb * dt_dy;
       if (val(ft) < 0.0) out = out + (-ft) * dt_dy;
-      const T avail = r_max(S.h[i4(li, lj)] - H_DRY, Z);
+      const T avail = r_max0(S.h[i4(li, lj)] - H_DRY);
       S.a[k] = (val(out) > val(avail) && val(out) > 0.0) ? dvp(avail, out) : cst<T>(1.0);
     }
     __syncthreads();
@@ -981,10 +1030,11 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, StageSmemT<T>& S,
       const int64_t g = (int64_t)gi * nc + gj;
       const int c4 = i4(li, lj), c3 = i3(li, lj);
       const T hc = S.h[c4];
-      const bool dc = val(hc) <= H_DRY;
+      const unsigned dryc = dry_window(S.dry[li + 4], lj - 1);
+      const bool dl = dryc & 1u, dc = dryc & 2u, dr = dryc & 4u;
+      const bool du = dry_window(S.dry[li + 3], lj) & 1u, dd = dry_window(S.dry[li + 5], lj) & 1u;
       T nh, nhu, nhv;
-      if (dc && (IN || (gi > 0 && gi + 1 < nr && gj > 0 && gj + 1 < nc)) && val(S.h[c4 - R4W]) <= H_DRY &&
-          val(S.h[c4 + R4W]) <= H_DRY && val(S.h[c4 - 1]) <= H_DRY && val(S.h[c4 + 1]) <= H_DRY) {
+      if (dc && (IN || (gi > 0 && gi + 1 < nr && gj > 0 && gj + 1 < nc)) && du && dd && dl && dr) {
         nh = hc;  // isolated-dry fast path (update.rs:1072-1088)
         nhu = Z;
         nhv = Z;
@@ -1009,9 +1059,7 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, StageSmemT<T>& S,
         const T dhv = (fxr_t - fxl_t) * dt_dx + (fyb_n - fyt_n) * dt_dy;
 
         double zfl, zfr, zft, zfb;
-        cell_face_beds<IN>(A, S.z, dc, val(S.h[c4 - 1]) <= H_DRY, val(S.h[c4 + 1]) <= H_DRY,
-                       val(S.h[c4 - R4W]) <= H_DRY, val(S.h[c4 + R4W]) <= H_DRY, c3, gi, gj, zfl,
-                       zfr, zft, zfb);
+        cell_face_beds<IN>(A, S.z, dc, dl, dr, du, dd, c3, gi, gj, zfl, zfr, zft, zfb);
 
         // Explicit bed-slope source on the reconstructed face states (update.rs:1140-1180).
         const double zc = S.z[c3];
@@ -1019,14 +1067,14 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, StageSmemT<T>& S,
         const T sex = S.sxe[isx(li, lj)];
         const T eta_left = (IN || gj > 0) ? eta_cell - sex : eta_cell;
         const T eta_right = (IN || gj + 1 < nc) ? eta_cell + sex : eta_cell;
-        const T hfl = r_max(eta_left - zfl, Z);
-        const T hfr = r_max(eta_right - zfr, Z);
+        const T hfl = r_max0(eta_left - zfl);
+        const T hfr = r_max0(eta_right - zfr);
         const T s_hu = over((hfl + hfr) * ((eta_left - hfl) - (eta_right - hfr)) * (0.5 * GRAVITY), A.rx);
         const T sey = S.sye[isy(li, lj)];
         const T eta_top = (IN || gi > 0) ? eta_cell - sey : eta_cell;
         const T eta_bot = (IN || gi + 1 < nr) ? eta_cell + sey : eta_cell;
-        const T hft = r_max(eta_top - zft, Z);
-        const T hfb = r_max(eta_bot - zfb, Z);
+        const T hft = r_max0(eta_top - zft);
+        const T hfb = r_max0(eta_bot - zfb);
         const T s_hv = over((hft + hfb) * ((eta_top - hft) - (eta_bot - hfb)) * (0.5 * GRAVITY), A.ry);
 
         if (val(new_h) <= H_VEL) {
