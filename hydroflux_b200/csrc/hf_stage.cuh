@@ -747,20 +747,11 @@ __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageS
   bool tile_mod = false;
   if constexpr (F64) tile_mod = S.extreme == 0;
   {
-    // ---- limited slopes: update.rs:459-540 (item k < SXN: x slope, else y)
-    auto slope_item = [&](int k, auto mod_tag) {
-      constexpr bool MOD = decltype(mod_tag)::value;
-      const bool xd = k < SXN;
-      int li, lj;
-      if (xd) {
-        const int r = k / SXW;
-        li = r - 1;
-        lj = k - r * SXW - 2;
-      } else {
-        const int kk = k - SXN, r = kk / SYW;
-        li = r - 2;
-        lj = kk - r * SYW - 1;
-      }
+    // ---- limited slopes: update.rs:459-540
+    auto slope_item = [&](int k, auto mod_tag, auto x_tag) {
+      constexpr bool MOD = decltype(mod_tag)::value, xd = decltype(x_tag)::value;
+      const int r = k / (xd ? SXW : SYW);
+      const int li = xd ? r - 1 : r - 2, lj = xd ? k - r * SXW - 2 : k - r * SYW - 1;
       const int gi = gi0 + li, gj = gj0 + lj;
       if (!IN && (gi < 0 || gi >= nr || gj < 0 || gj >= nc)) return;
       const int ga = xd ? gj : gi;
@@ -802,26 +793,18 @@ __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageS
         S.sxu[k] = su;
         S.sxv[k] = sv;
       } else {
-        S.sye[k - SXN] = se;
-        S.syu[k - SXN] = su;
-        S.syv[k - SXN] = sv;
+        S.sye[k] = se;
+        S.syu[k] = su;
+        S.syv[k] = sv;
       }
     };
 
-    // ---- faces: update.rs:676-728 (face beds), 890-926 (fluxes) (item k < FXN: x face)
-    auto face_item = [&](int k, auto mod_tag) {
-      constexpr bool MOD = decltype(mod_tag)::value;
-      const bool xd = k < FXN;
-      int li, lj;  // x face: (row li, face lj); y face: (face li, column lj)
-      if (xd) {
-        const int r = k / FXW;
-        li = r - 1;
-        lj = k - r * FXW - 1;
-      } else {
-        const int kk = k - FXN, r = kk / FYW;
-        li = r - 1;
-        lj = kk - r * FYW - 1;
-      }
+    // ---- faces: update.rs:676-728 (face beds), 890-926 (fluxes)
+    auto face_item = [&](int k, auto mod_tag, auto x_tag) {
+      constexpr bool MOD = decltype(mod_tag)::value, xd = decltype(x_tag)::value;
+      // x face: (row li, face lj); y face: (face li, column lj)
+      const int r = k / (xd ? FXW : FYW);
+      const int li = r - 1, lj = k - r * (xd ? FXW : FYW) - 1;
       const int gf = xd ? gj0 + lj : gi0 + li;  // face index along the normal
       const int na = xd ? nc : nr;
       const int gx = xd ? gi0 + li : gj0 + lj;  // index across
@@ -927,32 +910,39 @@ __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageS
       if (xd) {
         S.fxm[k] = m; S.fxnm[k] = nmn; S.fxnp[k] = npl; S.fxt[k] = tg;
       } else {
-        const int kk = k - FXN;
-        S.fym[kk] = m; S.fynm[kk] = nmn; S.fynp[kk] = npl; S.fyt[kk] = tg;
+        S.fym[k] = m; S.fynm[k] = nmn; S.fynp[k] = npl; S.fyt[k] = tg;
       }
     };
 
-    const std::true_type moderate{};
-    const std::false_type general{};
+    const std::true_type moderate{}, x{};
+    const std::false_type general{}, y{};
+    // x items, then y items from the thread after the last x item's on, so
+    // that the threads a partial pass leaves idle start with the y items.
+    auto pass = [&](auto item, int nx, int ny, auto mod_tag) {
+      for (int k = tid; k < nx; k += NTHREADS) item(k, mod_tag, x);
+      const int skip = nx % NTHREADS;
+      for (int k = tid >= skip ? tid - skip : tid - skip + NTHREADS; k < ny; k += NTHREADS)
+        item(k, mod_tag, y);
+    };
     if constexpr (F64) {
       if (tile_mod) {
-        for (int k = tid; k < SXN + SYN; k += NTHREADS) slope_item(k, moderate);
+        pass(slope_item, SXN, SYN, moderate);
         __syncthreads();
-        for (int k = tid; k < FXN + FYN; k += NTHREADS) face_item(k, moderate);
+        pass(face_item, FXN, FYN, moderate);
         __syncthreads();
       } else {
-        for (int k = tid; k < SXN + SYN; k += NTHREADS) slope_item(k, general);
+        pass(slope_item, SXN, SYN, general);
         __syncthreads();
         if (tid == 0) S.extreme = 0;  // read by all before the barrier above
-        for (int k = tid; k < FXN + FYN; k += NTHREADS) face_item(k, general);
+        pass(face_item, FXN, FYN, general);
         __syncthreads();
       }
     } else {  // slopes, x faces, then y faces (over the x momentum slopes)
-      for (int k = tid; k < SXN + SYN; k += NTHREADS) slope_item(k, general);
+      pass(slope_item, SXN, SYN, general);
       __syncthreads();
-      for (int k = tid; k < FXN; k += NTHREADS) face_item(k, general);
+      for (int k = tid; k < FXN; k += NTHREADS) face_item(k, general, x);
       __syncthreads();
-      for (int k = FXN + tid; k < FXN + FYN; k += NTHREADS) face_item(k, general);
+      for (int k = tid; k < FYN; k += NTHREADS) face_item(k, general, y);
       __syncthreads();
     }
     if constexpr (PF) {
