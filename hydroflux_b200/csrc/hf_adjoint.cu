@@ -41,7 +41,26 @@ struct AdjSmem {
   double lf4[FXN + FYN];    // face adjoint slots 4 and 5 (slots 0-3 live in the forward
   double lf5[FXN + FYN];    //   face arrays): x faces first, then y faces
   double lprim[3][R3N];     // adjoint of (eta, u, v)
+  unsigned char pick[SXN + SYN];  // which difference each limited slope took (slope_picks)
 };
+
+// The differences that the limited slopes of (eta, u, v) of a cell took, two
+// bits each: 0 none (the slope is the constant zero), 1 the left (upper) one,
+// 2 the right (lower) one; PICK_SKIP for a slope that passes no adjoint at all.
+constexpr unsigned PICK_SKIP = 0x80u;
+__device__ __forceinline__ unsigned pick_of(double l, double r, double d, bool mod) {
+  if (mod) {  // minmod_moderate's choice
+    if ((__double2hiint(l) ^ __double2hiint(r)) < 0 || l == 0.0 || r == 0.0) return 0u;
+    return fabs(l) < fabs(r) ? 1u : 2u;
+  }
+  return (unsigned)(minmod_pick(l, r, d) + 1);
+}
+// The derivative of a slope (times the spacing) by the cell at offset -o from
+// its own, for o = -1, 0, 1.
+__device__ __forceinline__ double pick_coef(unsigned pick, int o) {
+  const unsigned plus = o < 0 ? 2u : (o == 0 ? 1u : 3u), minus = o < 0 ? 3u : (o == 0 ? 2u : 1u);
+  return pick == plus ? 1.0 : (pick == minus ? -1.0 : 0.0);
+}
 
 // Which tile cells and faces exist: tile cell (li, lj) in [0,TY) x [0,TX).
 __device__ __forceinline__ bool in_tile(int li, int lj) {
@@ -119,10 +138,9 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stage_adj(const StageArgs A, co
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int tyi = tile / A.tiles_x;
     const int gi0 = tyi * TY, gj0 = (tile - tyi * A.tiles_x) * TX;
-    if (interior_tile(A, tile))
-      stage_tile_faces<double, false, true>(A, S, gi0, gj0, dt);
-    else
-      stage_tile_faces<double>(A, S, gi0, gj0, dt);
+    const bool mod = (interior_tile(A, tile)
+                          ? stage_tile_faces<double, false, true>(A, S, gi0, gj0, dt)
+                          : stage_tile_faces<double>(A, S, gi0, gj0, dt)) == TILE_MODERATE;
 
     // ---- A: per tile cell, epilogue / combination / update in reverse
     int src_lo = 0, src_hi = 0;
@@ -178,13 +196,13 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stage_adj(const StageArgs A, co
         eta_right = gj + 1 < nc ? eta_cell + sex : eta_cell;
         hfl = fmax(eta_left - zfl, 0.0);
         hfr = fmax(eta_right - zfr, 0.0);
-        const double s_hu = hfa::div_rn((hfl + hfr) * ((eta_left - hfl) - (eta_right - hfr)) * (0.5 * GRAVITY), dx);
+        const double s_hu = dvr((hfl + hfr) * ((eta_left - hfl) - (eta_right - hfr)) * (0.5 * GRAVITY), A.rx);
         sey = S.sye[isy(li, lj)];
         eta_top = gi > 0 ? eta_cell - sey : eta_cell;
         eta_bot = gi + 1 < nr ? eta_cell + sey : eta_cell;
         hft = fmax(eta_top - zft, 0.0);
         hfb = fmax(eta_bot - zfb, 0.0);
-        const double s_hv = hfa::div_rn((hft + hfb) * ((eta_top - hft) - (eta_bot - hfb)) * (0.5 * GRAVITY), dy);
+        const double s_hv = dvr((hft + hfb) * ((eta_top - hft) - (eta_bot - hfb)) * (0.5 * GRAVITY), A.ry);
         floor1 = new_h <= H_VEL;
         if (floor1) {
           nh = fmax(new_h, 0.0);
@@ -216,7 +234,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stage_adj(const StageArgs A, co
       if (A.finalize) {
         // forward values through friction and rain
         double fh = ch, fhu = chu, fhv = chv;
-        friction_cell<double>(fh, fhu, fhv, A.n[g], dt, A.dry_tol);
+        friction_moderate(fh, fhu, fhv, A.n[g], dt, A.dry_tol);
         double rh = fh;
         bool rain_zero = false;
         if (ctrl->rain_on) {
@@ -354,19 +372,12 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stage_adj(const StageArgs A, co
     __syncthreads();
 
     // ---- B3: faces in reverse; slots 0-5 replace the forward face values
-    for (int k = tid; k < FXN + FYN; k += NTHREADS) {
-      const bool xd = k < FXN;
-      const int kk = xd ? k : k - FXN;
-      int li, lj;
-      if (xd) {
-        const int r = kk / FXW;
-        li = r - 1;
-        lj = kk - r * FXW - 1;
-      } else {
-        const int r = kk / FYW;
-        li = r - 1;
-        lj = kk - r * FYW - 1;
-      }
+    // (moderate tiles with the unguarded quotients and roots)
+    auto face_rev = [&](int kk, auto mod_tag, auto x_tag) {
+      constexpr bool MOD = decltype(mod_tag)::value, xd = decltype(x_tag)::value;
+      const int k = xd ? kk : kk + FXN;
+      const int r = kk / (xd ? FXW : FYW);
+      const int li = r - 1, lj = kk - r * (xd ? FXW : FYW) - 1;
       double* f0 = xd ? S.fxm : S.fym;
       double* f1 = xd ? S.fxnm : S.fynm;
       double* f2 = xd ? S.fxnp : S.fynp;
@@ -453,8 +464,8 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stage_adj(const StageArgs A, co
               const double xp = (S.eta[p3] - se_p) - zf;
               const double h_m = fmax(xm, 0.0), h_p = fmax(xp, 0.0);
               double a0 = 0, a1 = 0, a2 = 0, b0 = 0, b1 = 0, b2 = 0;
-              wb_face_rev(h_m, h_m * un_m, h_m * ut_m, h_p, h_p * un_p, h_p * ut_p, zf, lm, ln1,
-                          ln2, lt, a0, a1, a2, b0, b1, b2);
+              wb_face_rev<MOD>(h_m, h_m * un_m, h_m * ut_m, h_p, h_p * un_p, h_p * ut_p, zf, lm,
+                               ln1, ln2, lt, a0, a1, a2, b0, b1, b2);
               // (h, h un, h ut) from (eta, un, ut): h = max(eta - zf, 0)
               s0 = (a0 + a1 * un_m + a2 * ut_m) * dmax0(xm);
               s1 = a1 * h_m;
@@ -469,8 +480,55 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stage_adj(const StageArgs A, co
       f0[kk] = s0; f1[kk] = s1; f2[kk] = s2; f3[kk] = s3;
       R.lf4[k] = s4;
       R.lf5[k] = s5;
+    };
+    {
+      const std::true_type x{};
+      const std::false_type y{};
+      auto pass = [&](auto mod_tag) {  // y items start with the threads x leaves idle
+        for (int k = tid; k < FXN; k += NTHREADS) face_rev(k, mod_tag, x);
+        const int skip = FXN % NTHREADS;
+        for (int k = tid >= skip ? tid - skip : tid - skip + NTHREADS; k < FYN; k += NTHREADS)
+          face_rev(k, mod_tag, y);
+      };
+      if (mod) pass(std::true_type{}); else pass(std::false_type{});
     }
     __syncthreads();
+
+    // ---- the picks of the limited slopes, once per slope: three cells read
+    // each (found again by every reader they took 950 of 6,400 warp
+    // instructions per warp of cells)
+    for (int k = tid; k < SXN + SYN; k += NTHREADS) {
+      const bool xd = k < SXN;
+      const int kk = xd ? k : k - SXN, r = kk / (xd ? SXW : SYW);
+      const int li = xd ? r - 1 : r - 2, lj = xd ? kk - r * SXW - 2 : kk - r * SYW - 1;
+      const int gi = gi0 + li, gj = gj0 + lj;
+      const int ga = xd ? gj : gi, na = xd ? nc : nr;
+      unsigned pick = PICK_SKIP;
+      if (gi >= 0 && gi < nr && gj >= 0 && gj < nc && na >= 2) {
+        bool anyd;
+        if (xd) {
+          anyd = (dry_window(S.dry[li + 4], lj - 2) & 31u) != 0;
+        } else {
+          const DryRow* d = &S.dry[li + 2];
+          const DryRow any{d[0].lo | d[1].lo | d[2].lo | d[3].lo | d[4].lo,
+                           d[0].hi | d[1].hi | d[2].hi | d[3].hi | d[4].hi};
+          anyd = (dry_window(any, lj) & 1u) != 0;
+        }
+        if (anyd) {
+        } else if (ga == 0) {
+          pick = 2u | 2u << 2 | 2u << 4;  // (q[+1] - q[0]) / d
+        } else if (ga == na - 1) {
+          pick = 1u | 1u << 2 | 1u << 4;  // (q[0] - q[-1]) / d
+        } else {
+          const int c3 = i3(li, lj), st = xd ? 1 : R3W;
+          const double d = xd ? dx : dy;
+          pick = pick_of(S.eta[c3] - S.eta[c3 - st], S.eta[c3 + st] - S.eta[c3], d, mod) |
+                 pick_of(S.u[c3] - S.u[c3 - st], S.u[c3 + st] - S.u[c3], d, mod) << 2 |
+                 pick_of(S.v[c3] - S.v[c3 - st], S.v[c3 + st] - S.v[c3], d, mod) << 4;
+        }
+      }
+      R.pick[k] = (unsigned char)pick;
+    }
 
     // ---- C1: per cell, gather the face adjoints into (eta, u, v) and slopes
     for (int k = tid; k < R3N; k += NTHREADS) {
@@ -561,54 +619,25 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stage_adj(const StageArgs A, co
       if (gi >= 0 && gi < nr && gj >= 0 && gj < nc) {
         double le = R.lprim[0][k], lu = R.lprim[1][k], lv = R.lprim[2][k];
         // slopes of this cell and its neighbours along x (o = -1, 0, 1) and y
+#pragma unroll
         for (int dir = 0; dir < 2; ++dir) {
           const bool xd = dir == 0;
-          const int na = xd ? nc : nr;
-          if (na < 2) continue;
-          const double d = xd ? dx : dy;
           const double inv_d = xd ? inv_dx : inv_dy;
+#pragma unroll
           for (int o = -1; o <= 1; ++o) {
             const int si = xd ? li : li + o, sj = xd ? lj + o : lj;  // slope cell
             const bool in_reg = xd ? (si >= -1 && si <= TY && sj >= -2 && sj <= TX + 1)
                                    : (si >= -2 && si <= TY + 1 && sj >= -1 && sj <= TX);
             if (!in_reg) continue;
-            const int ga = xd ? gj + o : gi + o;
-            if (ga < 0 || ga >= na) continue;
-            const int st4 = xd ? 1 : R4W, st3 = xd ? 1 : R3W;
-            const int s4 = i4(si, sj), s3 = i3(si, sj);
-            const int lo = max(ga - 2, 0) - ga, hi = min(ga + 2, na - 1) - ga;
-            bool anyd = false;
-            for (int w = lo; w <= hi; ++w) anyd |= S.h[s4 + w * st4] <= H_DRY;
-            if (anyd) continue;
             const int sidx = xd ? isx(si, sj) : isy(si, sj);
+            const unsigned pick = R.pick[xd ? sidx : SXN + sidx];
+            if (pick == PICK_SKIP) continue;
             const double Le = xd ? S.sxe[sidx] : S.sye[sidx];
             const double Lu = xd ? S.sxu[sidx] : S.syu[sidx];
             const double Lv = xd ? S.sxv[sidx] : S.syv[sidx];
-            // coefficient of this cell (offset -o from the slope cell) in each slope
-            const int rel = -o;  // -1: left neighbour of the slope cell, 0: itself, 1: right
-            double ce, cu, cv;
-            if (ga == 0) {  // (q[+1] - q[0]) / d
-              ce = cu = cv = rel == 1 ? 1.0 : (rel == 0 ? -1.0 : 0.0);
-            } else if (ga == na - 1) {  // (q[0] - q[-1]) / d
-              ce = cu = cv = rel == 0 ? 1.0 : (rel == -1 ? -1.0 : 0.0);
-            } else {
-              const double* fe = S.eta;
-              const double* fu = xd ? S.u : S.u;
-              const double* fv = xd ? S.v : S.v;
-              double cc[3];
-              const double* fld[3] = {fe, fu, fv};
-              for (int q = 0; q < 3; ++q) {
-                const double* F = fld[q];
-                const int pk = minmod_pick(F[s3] - F[s3 - st3], F[s3 + st3] - F[s3], d);
-                if (pk == 0) cc[q] = rel == 0 ? 1.0 : (rel == -1 ? -1.0 : 0.0);
-                else if (pk == 1) cc[q] = rel == 1 ? 1.0 : (rel == 0 ? -1.0 : 0.0);
-                else cc[q] = 0.0;
-              }
-              ce = cc[0]; cu = cc[1]; cv = cc[2];
-            }
-            le += ce * Le * inv_d;
-            lu += cu * Lu * inv_d;
-            lv += cv * Lv * inv_d;
+            le += pick_coef(pick & 3u, o) * Le * inv_d;
+            lu += pick_coef(pick >> 2 & 3u, o) * Lu * inv_d;
+            lv += pick_coef(pick >> 4 & 3u, o) * Lv * inv_d;
           }
         }
         // primitives: eta = h + z, u = hu / h, v = hv / h (when h > H_VEL)

@@ -27,9 +27,27 @@ namespace hf {
 // d max(x, 0) / dx with the Dual tie rule (dual.rs:130-141).
 HF_ADJ_HD double dmax0(double x) { return x > 0.0 ? 1.0 : (x < 0.0 ? 0.0 : 0.5); }
 
+// Quotients and roots of forward values in the reverse faces. MOD (the face of
+// a moderate tile): the unguarded forms, whose values are the same, with one
+// reciprocal per divisor. A face divides by six values, thirteen times.
+template <bool MOD> HF_ADJ_HD double rev_recip(double b) {
+  if (MOD && !hfa::low_word_ones(b)) return hfa::recip_rn(b);
+  return 1.0 / b;
+}
+template <bool MOD> HF_ADJ_HD double rev_quo(double a, double b, double y) {  // b > 0
+  return MOD ? hfa::quo_keep(a, b, y) : hfa::div_rn(a, b);
+}
+template <bool MOD> HF_ADJ_HD double rev_quo_neg(double a, double b, double y) {  // b < 0
+  return MOD ? hfa::quo_plus(a, b, y) : hfa::div_rn(a, b);
+}
+template <bool MOD> HF_ADJ_HD double rev_sqrt(double x) {
+  return MOD ? hfa::sqrt_rn_moderate(x) : sqrt(x);
+}
+
 // Reverse of hllc_normal: inputs are the forward arguments (values) and the
 // adjoint (Lm, Ln, Lt) of the outputs; the adjoint of the six arguments is
 // added to the L* references.
+template <bool MOD = false>
 HF_ADJ_HD void hllc_normal_rev(double h_l, double qn_l, double qt_l, double h_r,
                                                 double qn_r, double qt_r, double Lm, double Ln,
                                                 double Lt, double& L_hl, double& L_qnl,
@@ -38,10 +56,17 @@ HF_ADJ_HD void hllc_normal_rev(double h_l, double qn_l, double qt_l, double h_r,
   const bool wl = h_l > DRY_TOL;
   const bool wr = h_r > DRY_TOL;
   if (!wl && !wr) return;  // constant zero flux
-  const double cl = wl ? sqrt(h_l * GRAVITY) : 0.0;
-  const double cr = wr ? sqrt(h_r * GRAVITY) : 0.0;
-  const double un_l = wl ? hfa::div_rn(qn_l, h_l) : 0.0;
-  const double un_r = wr ? hfa::div_rn(qn_r, h_r) : 0.0;
+  double cl = 0.0, cr = 0.0, un_l = 0.0, un_r = 0.0, inv_hl = 0.0, inv_hr = 0.0;
+  if (wl) {
+    cl = rev_sqrt<MOD>(h_l * GRAVITY);
+    inv_hl = rev_recip<MOD>(h_l);
+    un_l = rev_quo<MOD>(qn_l, h_l, inv_hl);
+  }
+  if (wr) {
+    cr = rev_sqrt<MOD>(h_r * GRAVITY);
+    inv_hr = rev_recip<MOD>(h_r);
+    un_r = rev_quo<MOD>(qn_r, h_r, inv_hr);
+  }
   double sl, sr;
   if (wl && wr) {
     sl = fmin(un_l - cl, un_r - cr);
@@ -54,16 +79,18 @@ HF_ADJ_HD void hllc_normal_rev(double h_l, double qn_l, double qt_l, double h_r,
     sr = un_l + cl * 2.0;
   }
   bool left, star;
-  double s_star = 0.0, denom = 0.0;
+  double s_star = 0.0, denom = 0.0, inv_den = 0.0;
   if (sl >= 0.0) {
     left = true; star = false;
   } else if (sr <= 0.0) {
     left = false; star = false;
   } else {
     denom = h_r * (un_r - sr) - h_l * (un_l - sl);
-    s_star = fabs(denom) > 1.0e-12
-                 ? hfa::div_rn(h_r * (un_r - sr) * sl - h_l * (un_l - sl) * sr, denom)
-                 : (sl + sr) * 0.5;
+    s_star = (sl + sr) * 0.5;
+    if (fabs(denom) > 1.0e-12) {  // denom < 0 (wb_face_wet)
+      inv_den = rev_recip<MOD>(denom);
+      s_star = rev_quo_neg<MOD>(h_r * (un_r - sr) * sl - h_l * (un_l - sl) * sr, denom, inv_den);
+    }
     left = s_star >= 0.0;
     star = true;
   }
@@ -72,8 +99,6 @@ HF_ADJ_HD void hllc_normal_rev(double h_l, double qn_l, double qt_l, double h_r,
   const double qt = left ? qt_l : qt_r;
   const double un = left ? un_l : un_r;
   const bool wet = left ? wl : wr;
-  const double inv_hl = wl ? 1.0 / h_l : 0.0;
-  const double inv_hr = wr ? 1.0 / h_r : 0.0;
   const double inv_h = left ? inv_hl : inv_hr;
   const double ut = wet ? qt * inv_h : 0.0;
 
@@ -83,7 +108,7 @@ HF_ADJ_HD void hllc_normal_rev(double h_l, double qn_l, double qt_l, double h_r,
     // o = f + (hs - h) s, (hs s* - qn) s, (hs ut - qt) s; hs = h (s - un) / (s - s*)
     const double s = left ? sl : sr;
     const double D = s - s_star;
-    const double inv_D = 1.0 / D;
+    const double inv_D = rev_recip<MOD>(D);
     const double hs = h * (s - un) * inv_D;
     const double L_hs = Lm * s + Ln * s_star * s + Lt * ut * s;
     double L_s = Lm * (hs - h) + Ln * (hs * s_star - qn) + Lt * (hs * ut - qt);
@@ -120,7 +145,6 @@ HF_ADJ_HD void hllc_normal_rev(double h_l, double qn_l, double qt_l, double h_r,
     if (fabs(denom) > 1.0e-12) {
       // s* = (a1 sl - b1 sr) / (a1 - b1), a1 = h_r (un_r - sr), b1 = h_l (un_l - sl)
       const double a1 = h_r * (un_r - sr), b1 = h_l * (un_l - sl);
-      const double inv_den = 1.0 / denom;
       const double L_num = L_ss * inv_den;
       const double L_den = -L_ss * s_star * inv_den;
       const double L_a1 = L_num * sl + L_den;
@@ -171,6 +195,7 @@ HF_ADJ_HD void hllc_normal_rev(double h_l, double qn_l, double qt_l, double h_r,
 
 // Reverse of wb_face: adjoint (L_mass, L_nm, L_np, L_t) of the outputs to the
 // adjoint of the oriented states (added to the L* references).
+template <bool MOD = false>
 HF_ADJ_HD void wb_face_rev(double hL, double qnL, double qtL, double hR,
                                             double qnR, double qtR, double zf, double L_mass,
                                             double L_nm, double L_np, double L_t, double& LhL,
@@ -180,13 +205,16 @@ HF_ADJ_HD void wb_face_rev(double hL, double qnL, double qtL, double hR,
   const double xL = hL + zf - z_max, xR = hR + zf - z_max;
   const double hsL = fmax(xL, 0.0), hsR = fmax(xR, 0.0);
   double unL = 0.0, utL = 0.0, unR = 0.0, utR = 0.0;
+  double inv_hL = 0.0, inv_hR = 0.0;
   if (hL > H_VEL) {
-    unL = hfa::div_rn(qnL, hL);
-    utL = hfa::div_rn(qtL, hL);
+    inv_hL = rev_recip<MOD>(hL);
+    unL = rev_quo<MOD>(qnL, hL, inv_hL);
+    utL = rev_quo<MOD>(qtL, hL, inv_hL);
   }
   if (hR > H_VEL) {
-    unR = hfa::div_rn(qnR, hR);
-    utR = hfa::div_rn(qtR, hR);
+    inv_hR = rev_recip<MOD>(hR);
+    unR = rev_quo<MOD>(qnR, hR, inv_hR);
+    utR = rev_quo<MOD>(qtR, hR, inv_hR);
   }
   // corr = (h^2 - hs^2) g/2 enters n_minus (left) and n_plus (right)
   LhL += L_nm * (2.0 * hL) * (0.5 * GRAVITY);
@@ -194,23 +222,23 @@ HF_ADJ_HD void wb_face_rev(double hL, double qnL, double qtL, double hR,
   double L_hsL = -L_nm * (2.0 * hsL) * (0.5 * GRAVITY);
   double L_hsR = -L_np * (2.0 * hsR) * (0.5 * GRAVITY);
   double a0 = 0.0, a1 = 0.0, a2 = 0.0, b0 = 0.0, b1 = 0.0, b2 = 0.0;
-  hllc_normal_rev(hsL, hsL * unL, hsL * utL, hsR, hsR * unR, hsR * utR, L_mass, L_nm + L_np, L_t,
+  hllc_normal_rev<MOD>(hsL, hsL * unL, hsL * utL, hsR, hsR * unR, hsR * utR, L_mass, L_nm + L_np, L_t,
                   a0, a1, a2, b0, b1, b2);
   L_hsL += a0 + a1 * unL + a2 * utL;
   L_hsR += b0 + b1 * unR + b2 * utR;
   LhL += L_hsL * dmax0(xL);
   LhR += L_hsR * dmax0(xR);
   if (hL > H_VEL) {  // qns = hs * (qn / h)
-    const double LunL = a1 * hsL, LutL = a2 * hsL, inv = 1.0 / hL;
-    LqnL += LunL * inv;
-    LqtL += LutL * inv;
-    LhL -= (LunL * unL + LutL * utL) * inv;
+    const double LunL = a1 * hsL, LutL = a2 * hsL;
+    LqnL += LunL * inv_hL;
+    LqtL += LutL * inv_hL;
+    LhL -= (LunL * unL + LutL * utL) * inv_hL;
   }
   if (hR > H_VEL) {
-    const double LunR = b1 * hsR, LutR = b2 * hsR, inv = 1.0 / hR;
-    LqnR += LunR * inv;
-    LqtR += LutR * inv;
-    LhR -= (LunR * unR + LutR * utR) * inv;
+    const double LunR = b1 * hsR, LutR = b2 * hsR;
+    LqnR += LunR * inv_hR;
+    LqtR += LutR * inv_hR;
+    LhR -= (LunR * unR + LutR * utR) * inv_hR;
   }
 }
 
