@@ -495,7 +495,7 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stage_adj(const StageArgs A, co
     __syncthreads();
 
     // ---- the picks of the limited slopes, once per slope: three cells read
-    // each (found again by every reader they took 950 of 6,400 warp
+    // each (found again by every reader they took 1,900 of 6,800 warp
     // instructions per warp of cells)
     for (int k = tid; k < SXN + SYN; k += NTHREADS) {
       const bool xd = k < SXN;
