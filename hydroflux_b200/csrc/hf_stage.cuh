@@ -243,6 +243,11 @@ struct StagePfSmem {
   StageSmem s;
   alignas(16) double hst[R4N];
 };
+// Depth buffers of a run of dry tiles (stage_dry_run), over the slopes, faces
+// and alpha that such tiles do not use.
+constexpr int DRY_RING = 4;
+static_assert(sizeof(StageSmem) - offsetof(StageSmem, sxe) >= (DRY_RING * R4N + 1) * sizeof(double),
+              "the ring fits over the slopes and faces");
 static_assert(R3W % 2 == 0 && R4W % 2 == 0 && TX % 2 == 0, "column pairs");
 static_assert(offsetof(StageSmem, h) % 16 == 0 && offsetof(StageSmem, eta) % 16 == 8 &&
                   offsetof(StageSmem, u) % 16 == 8 && offsetof(StageSmem, v) % 16 == 8 &&
@@ -259,14 +264,17 @@ static_assert(offsetof(StageSmem, h) % 16 == 0 && offsetof(StageSmem, eta) % 16 
 // outside the grid). The 3-cell halo rows (columns gj0-3 .. gj0+TX+2) take
 // TX/2 + 1 pairs and one single column at each end. Otherwise every element
 // is copied alone.
-__device__ __forceinline__ void stage_prefetch(const StageArgs& A, StageSmem& S, double* hst,
-                                               int tile) {
+__device__ __forceinline__ bool copies_pairs(const StageArgs& A) {
+  const uintptr_t any = (uintptr_t)A.in_h | (uintptr_t)A.z | (uintptr_t)A.in_hu |
+                        (uintptr_t)A.in_hv;
+  return ((A.nc & 1) | (int)(any & 15)) == 0;
+}
+// The depths of a tile into hst.
+__device__ __forceinline__ void stage_prefetch_h(const StageArgs& A, double* hst, int tile) {
   const int nr = A.nr, nc = A.nc;
   const int tyi = tile / A.tiles_x;
   const int gi0 = tyi * TY, gj0 = (tile - tyi * A.tiles_x) * TX;
-  const uintptr_t any = (uintptr_t)A.in_h | (uintptr_t)A.z | (uintptr_t)A.in_hu |
-                        (uintptr_t)A.in_hv;
-  if (((nc & 1) | (int)(any & 15)) == 0) {
+  if (copies_pairs(A)) {
     constexpr int PW = R4W / 2;  // pairs per 4-cell halo row
     for (int k = threadIdx.x; k < R4H * PW; k += NTHREADS) {
       const int r = k / PW, cc = 2 * (k - r * PW);
@@ -274,6 +282,36 @@ __device__ __forceinline__ void stage_prefetch(const StageArgs& A, StageSmem& S,
       const bool real = gi >= 0 && gi < nr && gj >= 0 && gj < nc;
       cp_async16(&hst[r * R4W + cc], A.in_h + (real ? (int64_t)gi * nc + gj : 0), real);
     }
+  } else {
+    for (int k = threadIdx.x; k < R4N; k += NTHREADS) {
+      const int r = k / R4W, cc = k - r * R4W;
+      const int gi = gi0 + r - 4, gj = gj0 + cc - 4;
+      const bool real = gi >= 0 && gi < nr && gj >= 0 && gj < nc;
+      cp_async8(&hst[k], A.in_h + (real ? (int64_t)gi * nc + gj : 0), real);
+    }
+  }
+  asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+// Whether the depths that this thread copied with stage_prefetch_h (and waited
+// for) are all dry.
+__device__ __forceinline__ bool prefetched_dry(const StageArgs& A, const double* hst) {
+  bool dry = true;
+  if (copies_pairs(A)) {
+    for (int k = threadIdx.x; k < R4N / 2; k += NTHREADS) {
+      const double2 h = reinterpret_cast<const double2*>(hst)[k];
+      dry = dry && h.x <= H_DRY && h.y <= H_DRY;
+    }
+  } else {
+    for (int k = threadIdx.x; k < R4N; k += NTHREADS) dry = dry && hst[k] <= H_DRY;
+  }
+  return dry;
+}
+// Its bed and momenta into S.eta, S.u, S.v.
+__device__ __forceinline__ void stage_prefetch_rest(const StageArgs& A, StageSmem& S, int tile) {
+  const int nr = A.nr, nc = A.nc;
+  const int tyi = tile / A.tiles_x;
+  const int gi0 = tyi * TY, gj0 = (tile - tyi * A.tiles_x) * TX;
+  if (copies_pairs(A)) {
     constexpr int NP = (R3W - 2) / 2;  // pairs per 3-cell halo row (columns 2 .. R3W-1)
     for (int k = threadIdx.x; k < R3H * (NP + 2); k += NTHREADS) {
       const int r3 = k / (NP + 2), j = k - r3 * (NP + 2);
@@ -292,23 +330,23 @@ __device__ __forceinline__ void stage_prefetch(const StageArgs& A, StageSmem& S,
         cp_async8(&S.v[k3], A.in_hv + g, real);
       }
     }
-    asm volatile("cp.async.commit_group;\n" ::: "memory");
-    return;
-  }
-  for (int k = threadIdx.x; k < R4N; k += NTHREADS) {
-    const int r = k / R4W, cc = k - r * R4W;
-    const int gi = gi0 + r - 4, gj = gj0 + cc - 4;
-    const bool real = gi >= 0 && gi < nr && gj >= 0 && gj < nc;
-    const int64_t g = real ? (int64_t)gi * nc + gj : 0;
-    cp_async8(&hst[k], A.in_h + g, real);
-    if (r >= 1 && r < R4H - 1 && cc >= 1 && cc < R4W - 1) {
-      const int k3 = (r - 1) * R3W + (cc - 1);
+  } else {
+    for (int k3 = threadIdx.x; k3 < R3N; k3 += NTHREADS) {
+      const int r3 = k3 / R3W, cc = k3 - r3 * R3W;
+      const int gi = gi0 + r3 - 3, gj = gj0 + cc - 3;
+      const bool real = gi >= 0 && gi < nr && gj >= 0 && gj < nc;
+      const int64_t g = real ? (int64_t)gi * nc + gj : 0;
       cp_async8(&S.eta[k3], A.z + g, real);
       cp_async8(&S.u[k3], A.in_hu + g, real);
       cp_async8(&S.v[k3], A.in_hv + g, real);
     }
   }
   asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+__device__ __forceinline__ void stage_prefetch(const StageArgs& A, StageSmem& S, double* hst,
+                                               int tile) {
+  stage_prefetch_h(A, hst, tile);
+  stage_prefetch_rest(A, S, tile);
 }
 
 // ---------------------------------------------------------------------------
@@ -633,7 +671,7 @@ __device__ __forceinline__ bool moderate_cell(double h, double z, double hu, dou
   return __double2hiint(h) >= 0 && hfa::moderate_or_zero(h) && hfa::moderate_or_zero(z) &&
          hfa::moderate_or_zero(hu) && hfa::moderate_or_zero(hv);
 }
-template <class T, bool PF = false, bool IN = false, bool DRY = false>
+template <class T, bool PF = false, bool IN = false, bool DRY = false, bool HD = false>
 __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageSmemT<T>& S, int gi0,
                                                  int gj0, double dt, double* hst = nullptr,
                                                  int next = -1,
@@ -685,7 +723,9 @@ __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageS
     if (!mod) S.extreme = 1;
     if constexpr (SKIP) {
       if (__syncthreads_and(dry)) {
-        if (next >= 0) stage_prefetch(next_args ? *next_args : A, S, hst, next);
+        if constexpr (!HD) {
+          if (next >= 0) stage_prefetch(next_args ? *next_args : A, S, hst, next);
+        }
         return TILE_DRY;
       }
     } else {
@@ -946,8 +986,9 @@ __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageS
       __syncthreads();
     }
     if constexpr (PF) {
-      if (next >= 0)  // eta, u, v and hst are dead now
+      if (next >= 0) {  // eta, u, v and hst are dead now
         stage_prefetch(next_args ? *next_args : A, S, hst, next);
+      }
     }
 
     // ---- alpha mass rescaling factors: update.rs:953-982 (tile + 1-cell ring)
@@ -977,11 +1018,14 @@ __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageS
 // finalize epilogue into (sxm, sym, nonfin).
 // IN: the tile and its 4-cell halo lie inside the grid (no side is reached),
 // so the boundary branches compile away; the arithmetic is the same.
-template <class T, bool PF = false, bool IN = false>
-__device__ __forceinline__ void stage_tile(const StageArgs& A, StageSmemT<T>& S, int tile,
-                                           double& sxm, double& sym, unsigned long long& nonfin,
-                                           double* hst = nullptr, int next = -1,
-                                           const StageArgs* next_args = nullptr) {
+// HD: nothing is copied for the next tile when this one is dry (the caller
+// goes on with stage_dry_run).
+template <class T, bool PF = false, bool IN = false, bool HD = false>
+__device__ __forceinline__ TileClass stage_tile(const StageArgs& A, StageSmemT<T>& S, int tile,
+                                                double& sxm, double& sym,
+                                                unsigned long long& nonfin, double* hst = nullptr,
+                                                int next = -1,
+                                                const StageArgs* next_args = nullptr) {
   Ctrl* ctrl = A.ctrl;
   const double dt = ctrl->dt;
   const int nr = A.nr, nc = A.nc;
@@ -994,8 +1038,9 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, StageSmemT<T>& S,
     const int tyi = tile / A.tiles_x;
     const int gi0 = tyi * TY, gj0 = (tile - tyi * A.tiles_x) * TX;
     // Dry interior tiles skip their slopes, faces and alpha (f64 forward stage).
-    const bool mod = stage_tile_faces<T, PF, IN, std::is_same<T, double>::value>(
-                         A, S, gi0, gj0, dt, hst, next, next_args) == TILE_MODERATE;
+    const TileClass cls = stage_tile_faces<T, PF, IN, std::is_same<T, double>::value, HD>(
+        A, S, gi0, gj0, dt, hst, next, next_args);
+    const bool mod = cls == TILE_MODERATE;
     // A source term's division by the spacing (moderate tiles: unguarded).
     auto over = [mod](T a, const hfa::RecipD& r) -> T {
       if constexpr (std::is_same<T, double>::value) {
@@ -1105,6 +1150,49 @@ __device__ __forceinline__ void stage_tile(const StageArgs& A, StageSmemT<T>& S,
       Field<T>::st(A.out_hv, A.tan.out_hv, g, nhv);
     }
     __syncthreads();
+    return cls;
+  }
+}
+
+// The stage of an interior tile whose depths (hst, with the halo) are all dry:
+// every cell takes the isolated-dry update (update.rs:1072-1088). un_h0: U^n's
+// depth of the thread's first cell, loaded ahead.
+__device__ __forceinline__ void stage_tile_dry(const StageArgs& A, const double* hst, int tile,
+                                               double un_h0, double& sxm, double& sym,
+                                               unsigned long long& nonfin) {
+  const Ctrl* ctrl = A.ctrl;
+  const int tyi = tile / A.tiles_x;
+  const int gi0 = tyi * TY, gj0 = (tile - tyi * A.tiles_x) * TX;
+  int src_lo = 0, src_hi = 0;
+  if (A.finalize && A.f.n_src > 0) {
+    const int b = source_bucket(tile, A.tiles_x);
+    src_lo = A.f.tile_start[b];
+    src_hi = A.f.tile_start[b + 1];
+  }
+  for (int q = 0; q < CELLS_PER_THREAD; ++q) {
+    const int li = threadIdx.x / TX + ROWS_PER_PASS * q, lj = threadIdx.x % TX;
+    if (kPartialPass && li >= TY) continue;
+    const int gi = gi0 + li, gj = gj0 + lj;
+    const int64_t g = (int64_t)gi * A.nc + gj;
+    double nh = hst[i4(li, lj)], nhu = 0.0, nhv = 0.0;
+    if (A.combine) {
+      nh = ((q == 0 ? un_h0 : A.un_h[g]) + nh) * 0.5;
+      if (nh <= H_VEL) {
+        nh = r_max(nh, 0.0);
+      } else {
+        nhu = (A.un_hu[g] + nhu) * 0.5;
+        nhv = (A.un_hv[g] + nhv) * 0.5;
+      }
+    }
+    if (A.finalize) {
+      if (!(nh <= A.dry_tol)) friction_moderate(nh, nhu, nhv, A.n[g], ctrl->dt, A.dry_tol);
+      forcings_cell<double>(A, ctrl, gi, gj, A.f.tile_order, src_lo, src_hi, nh, nhu, nhv);
+      cfl_cell<true>(A, gi, gj, g, nh, nhu, nhv, sxm, sym);
+      if (ctrl->check_finite && !isfinite(nh)) ++nonfin;
+    }
+    A.out_h[g] = nh;
+    A.out_hu[g] = nhu;
+    A.out_hv[g] = nhv;
   }
 }
 
@@ -1114,6 +1202,41 @@ __device__ __forceinline__ bool interior_tile(const StageArgs& A, int tile) {
   const int tyi = tile / A.tiles_x;
   const int gi0 = tyi * TY, gj0 = (tile - tyi * A.tiles_x) * TX;
   return gi0 >= 4 && gj0 >= 4 && gi0 + TY + 4 <= A.nr && gj0 + TX + 4 <= A.nc;
+}
+
+// After a dry tile: the stage of the tiles that follow with stride `stride`
+// while they are interior and dry. Each is known by its depths, which are
+// copied up to three tiles ahead, and loads no bed, momentum or Manning value;
+// one barrier per tile. Returns the first tile left, of which nothing is in
+// flight. (All dry at 2048^2: 315 -> 218 us a step; with 15% of the tiles wet
+// 356 -> 277.)
+__device__ __forceinline__ int stage_dry_run(const StageArgs& A, StageSmem& S, int tile, int ntiles,
+                                             int stride, double& sxm, double& sym,
+                                             unsigned long long& nonfin) {
+  double* ring = reinterpret_cast<double*>(
+      (reinterpret_cast<uintptr_t>(&S.sxe[0]) + 15) & ~(uintptr_t)15);
+  auto fetch = [&](int slot, int t) {
+    if (t < ntiles) stage_prefetch_h(A, ring + slot * R4N, t);
+    else asm volatile("cp.async.commit_group;\n" ::: "memory");
+  };
+  for (int j = 0; j < DRY_RING - 1; ++j) fetch(j, tile + j * stride);
+  const int li = threadIdx.x / TX, lj = threadIdx.x % TX;
+  for (int slot = 0; tile < ntiles; tile += stride, slot = slot + 1 == DRY_RING ? 0 : slot + 1) {
+    const bool in = interior_tile(A, tile);
+    double un_h0 = 0.0;
+    if (A.combine && in && li < TY) {
+      const int tyi = tile / A.tiles_x;
+      un_h0 = A.un_h[(int64_t)(tyi * TY + li) * A.nc + (tile - tyi * A.tiles_x) * TX + lj];
+    }
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(DRY_RING - 2) : "memory");
+    if (!__syncthreads_and(in && prefetched_dry(A, ring + slot * R4N))) break;
+    // every thread is done with the tile before: its slot takes the next copy
+    fetch(slot == 0 ? DRY_RING - 1 : slot - 1, tile + (DRY_RING - 1) * stride);
+    stage_tile_dry(A, ring + slot * R4N, tile, un_h0, sxm, sym, nonfin);
+  }
+  cp_async_wait_all();
+  __syncthreads();  // the ring's memory is the next tile's slopes and faces
+  return tile;
 }
 
 }  // namespace HF_GEOM

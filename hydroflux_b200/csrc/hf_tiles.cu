@@ -121,14 +121,20 @@ __global__ void __launch_bounds__(NTHREADS, HF_MIN_BLOCKS) k_stage_pf(const Stag
   unsigned long long nonfin = 0;
   if (threadIdx.x == 0) P.s.extreme = 0;
   if ((int)blockIdx.x < ntiles) stage_prefetch(A, P.s, P.hst, blockIdx.x);
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+  int tile = blockIdx.x;
+  while (tile < ntiles) {
     cp_async_wait_all();
     __syncthreads();
     const int next = tile + (int)gridDim.x < ntiles ? tile + (int)gridDim.x : -1;
-    if (interior_tile(A, tile))
-      stage_tile<double, true, true>(A, P.s, tile, sxm, sym, nonfin, P.hst, next);
-    else
-      stage_tile<double, true>(A, P.s, tile, sxm, sym, nonfin, P.hst, next);
+    const TileClass cls =
+        interior_tile(A, tile)
+            ? stage_tile<double, true, true, true>(A, P.s, tile, sxm, sym, nonfin, P.hst, next)
+            : stage_tile<double, true, false, true>(A, P.s, tile, sxm, sym, nonfin, P.hst, next);
+    tile += (int)gridDim.x;
+    if (cls == TILE_DRY && tile < ntiles) {
+      tile = stage_dry_run(A, P.s, tile, ntiles, gridDim.x, sxm, sym, nonfin);
+      if (tile < ntiles) stage_prefetch(A, P.s, P.hst, tile);
+    }
   }
   if (A.finalize) {
     block_reduce_speeds(sxm, sym, nonfin, A.ctrl);
