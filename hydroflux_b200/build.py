@@ -17,7 +17,7 @@ ROOT = os.path.dirname(HERE)
 INCLUDE = os.path.join(ROOT, "include")
 OUT = os.path.join(HERE, "libhydroflux_gpu.so")
 
-SOURCES = ["hf_kernels.cu", "hf_tiles.cu", "hf_api.cu", "hf_noalloc.cu", "hf_batch.cu",
+SOURCES = ["hf_kernels.cu", "hf_tiles.cu", "hf_dual.cu", "hf_api.cu", "hf_noalloc.cu", "hf_batch.cu",
            "hf_serve.cu", "hf_adjoint.cu", "hf_calib.cu", "hf_io.cu"]
 # hf_tiles.cu is compiled once more for each other tile geometry (the default
 # macros give 32 x 8 tiles by 256 threads; see hf_internal.h).
@@ -27,6 +27,9 @@ GEOMETRIES = [("hf_tiles.cu", "hf_tiles_%s.o" % name,
               for name, index, rows, threads, blocks in (
                   ("g32", 1, 32, 1024, 1), ("g8w", 2, 8, 768, 1), ("g8m", 3, 8, 384, 2),
                   ("g4", 4, 4, 512, 1))]
+GEOMETRIES.append(("hf_dual.cu", "hf_dual_g8d.o",
+                   ["-DHF_GEOM=g8d", "-DHF_GEOM_INDEX=5", "-DHF_TILE_Y=8", "-DHF_THREADS=512",
+                    "-DHF_MIN_BLOCKS=1"]))
 GENCODE = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--fmad=false", "-prec-div=true",
               "-prec-sqrt=true", "-Xcompiler", "-fPIC", "-Xcompiler", "-O2",

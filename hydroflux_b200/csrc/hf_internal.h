@@ -38,7 +38,7 @@ namespace hf {
 // All compute every cell with the same operations: results are identical.
 constexpr int TX = 32;
 constexpr int kGeomSmall = 0, kGeomLarge = 1, kGeomWide = 2, kGeomMid = 3, kGeomLow = 4;
-constexpr int kGeomTileH[5] = {8, 32, 8, 8, 4};
+constexpr int kGeomTileH[6] = {8, 32, 8, 8, 4, 8};  // the last: the wide tangent CTA (hf_dual.cu)
 constexpr int kLargeTilesMin = 100;
 // A scenario of an ensemble or server with at least this many 32 x 32 tiles
 // (about 3.5 waves of the 148 SMs; from 724 x 724 cells on) fills the GPU
@@ -230,6 +230,12 @@ struct StageArgs {
   ForcingDev f;
   TanPtrs tan;   // DualD kernels only
 };
+
+// SMs of the current device.
+int64_t sm_count();
+// The tangent stage on 512-thread CTAs (hf_dual.cu).
+void dual_wide_prepare();
+void launch_stage_dual_wide(const StageArgs& a, int grid, void* stream, int lanes);
 
 // Launchers of the step control and standalone kernels (hf_kernels.cu).
 int launch_control(Ctrl* ctrl, double dx, double dy, const ForcingDev& f, void* stream);

@@ -346,7 +346,6 @@ int geom_for(int64_t nr, int64_t nc) {
   return t >= kLargeTilesMin ? kGeomLarge : kGeomSmall;
 }
 
-namespace {
 int64_t sm_count() {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -354,7 +353,6 @@ int64_t sm_count() {
     cudaGetLastError();
   return sms > 0 ? sms : 148;
 }
-}  // namespace
 
 bool small_tiles_pay(int64_t n8, int64_t n32) {
   const int64_t sms = sm_count(), w8 = (n8 + 3 * sms - 1) / (3 * sms);

@@ -1239,5 +1239,26 @@ __device__ __forceinline__ int stage_dry_run(const StageArgs& A, StageSmem& S, i
   return tile;
 }
 
+// The arguments of tangent lane `lane`: its tangent arrays, and no value
+// outputs unless it is lane 0 (the values are the same in every lane).
+__device__ __forceinline__ void lane_args(const StageArgs& A, int lane, StageArgs& L) {
+  L = A;
+  if (lane == 0) return;
+  const long long o = (long long)lane * A.tan.lane_stride;
+  auto shift = [o](const double* p) { return p ? p + o : p; };
+  auto shift_w = [o](double* p) { return p ? p + o : p; };
+  L.tan.in_h = shift(A.tan.in_h);
+  L.tan.in_hu = shift(A.tan.in_hu);
+  L.tan.in_hv = shift(A.tan.in_hv);
+  L.tan.out_h = shift_w(A.tan.out_h);
+  L.tan.out_hu = shift_w(A.tan.out_hu);
+  L.tan.out_hv = shift_w(A.tan.out_hv);
+  L.tan.un_h = shift(A.tan.un_h);
+  L.tan.un_hu = shift(A.tan.un_hu);
+  L.tan.un_hv = shift(A.tan.un_hv);
+  L.tan.n = shift(A.tan.n);
+  L.out_h = L.out_hu = L.out_hv = nullptr;
+}
+
 }  // namespace HF_GEOM
 }  // namespace hf

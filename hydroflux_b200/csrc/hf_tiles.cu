@@ -6,12 +6,11 @@
 // phases are in hf_stage.cuh). This file holds the kernels whose work is cut
 // into those tiles -- the single-grid stage (k_stage_pf), the ensemble stage
 // (k_stage_batch), the forward-Euler finalize and the CFL reductions -- and
-// their launchers. The build compiles it twice: with the 32 x 8 geometry
-// (namespace g8, 256 threads, three CTAs per SM), which also carries the
-// strip kernel and the DualD tangent kernels, and with the 32 x 32 geometry
-// (namespace g32, 1024 threads, one CTA per SM). The geometry's symbols live
-// in its inline namespace, so both builds link into one library; the host
-// code reaches the one a grid uses through geom_ops().
+// their launchers. The build compiles it once per geometry (hf_internal.h); the
+// 32 x 8 one with 256 threads (namespace g8) also carries the strip kernel and
+// the DualD finalize. A geometry's symbols live in its inline namespace, so the
+// builds link into one library; the host code reaches the one a grid uses
+// through geom_ops().
 #include <cuda_runtime.h>
 
 #include <type_traits>
@@ -40,73 +39,6 @@ struct DevGuard {
   }
 };
 }  // namespace
-
-// Blocks per SM the stage kernel is compiled for: in the 32 x 8 geometry the
-// f64 tile takes 71 KB of shared memory (three CTAs per SM) and the DualD
-// tile 112 KB (two); in the 32 x 32 geometry the f64 tile takes 211 KB (one).
-template <class T> struct StageOcc { static constexpr int value = HF_MIN_BLOCKS; };
-template <> struct StageOcc<DualD> { static constexpr int value = 2; };
-
-// The arguments of tangent lane `lane`: its tangent arrays, and no value
-// outputs unless it is lane 0 (the values are the same in every lane).
-__device__ void lane_args(const StageArgs& A, int lane, StageArgs& L) {
-  L = A;
-  if (lane == 0) return;
-  const long long o = (long long)lane * A.tan.lane_stride;
-  auto shift = [o](const double* p) { return p ? p + o : p; };
-  auto shift_w = [o](double* p) { return p ? p + o : p; };
-  L.tan.in_h = shift(A.tan.in_h);
-  L.tan.in_hu = shift(A.tan.in_hu);
-  L.tan.in_hv = shift(A.tan.in_hv);
-  L.tan.out_h = shift_w(A.tan.out_h);
-  L.tan.out_hu = shift_w(A.tan.out_hu);
-  L.tan.out_hv = shift_w(A.tan.out_hv);
-  L.tan.un_h = shift(A.tan.un_h);
-  L.tan.un_hu = shift(A.tan.un_hu);
-  L.tan.un_hv = shift(A.tan.un_hv);
-  L.tan.n = shift(A.tan.n);
-  L.out_h = L.out_hu = L.out_hv = nullptr;
-}
-
-#if HF_GEOM_PRIMARY
-template <class T>
-__device__ __forceinline__ void stage_tile_any(const StageArgs& A, StageSmemT<T>& S, int tile,
-                                               double& sxm, double& sym,
-                                               unsigned long long& nonfin) {
-  if (interior_tile(A, tile))
-    stage_tile<T, false, true>(A, S, tile, sxm, sym, nonfin);
-  else
-    stage_tile<T>(A, S, tile, sxm, sym, nonfin);
-}
-
-// One stage of one grid over a persistent tile loop. For T = DualD,
-// blockIdx.y is the tangent lane (vector mode); the CFL reduction and the
-// clock belong to lane 0.
-template <class T>
-__global__ void __launch_bounds__(NTHREADS, StageOcc<T>::value) k_stage(const StageArgs A) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  StageSmemT<T>& S = *reinterpret_cast<StageSmemT<T>*>(smem_raw);
-  if (!A.ctrl->active) return;
-  const int ntiles = A.tiles_x * A.tiles_y;
-  double sxm = 0.0, sym = 0.0;
-  unsigned long long nonfin = 0;
-  if constexpr (std::is_same<T, DualD>::value) {
-    __shared__ __align__(16) unsigned char lane_raw[sizeof(StageArgs)];
-    StageArgs& L = *reinterpret_cast<StageArgs*>(lane_raw);
-    if (threadIdx.x == 0) lane_args(A, blockIdx.y, L);
-    __syncthreads();
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-      stage_tile_any<T>(L, S, tile, sxm, sym, nonfin);
-  } else {
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x)
-      stage_tile_any<T>(A, S, tile, sxm, sym, nonfin);
-  }
-  if (A.finalize && blockIdx.y == 0) {
-    block_reduce_speeds(sxm, sym, nonfin, A.ctrl);
-    if (blockIdx.x == 0 && threadIdx.x == 0) commit_clock(A.ctrl);
-  }
-}
-#endif  // HF_GEOM_PRIMARY
 
 // The f64 stage of one grid, software-pipelined: while a CTA computes the
 // alpha and update phases of one tile, the raw inputs of its next tile are
@@ -527,36 +459,8 @@ int launch_stage_strip(const StageArgs& a, const StripMaps& m, int grid, void* s
   return launched(stream);
 }
 
-int stage_dual_grid_size(int tiles, int device) {
-  static int cached[64] = {0};
-  int per_sm = 0, sms = 0;
-  if (device >= 0 && device < 64 && cached[device] > 0) {
-    per_sm = cached[device];
-  } else {
-    DevGuard dg(device);
-    cudaFuncSetAttribute(k_stage<DualD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)sizeof(StageSmemT<DualD>));
-    // two 112 KB tiles per SM need the largest shared-memory carveout
-    cudaFuncSetAttribute(k_stage<DualD>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                         (int)cudaSharedmemCarveoutMaxShared);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage<DualD>, NTHREADS,
-                                                  sizeof(StageSmemT<DualD>));
-    if (per_sm < 1) per_sm = 1;
-    if (device >= 0 && device < 64) cached[device] = per_sm;
-  }
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  int g = per_sm * (sms > 0 ? sms : 148);
-  return tiles < g ? (tiles < 1 ? 1 : tiles) : g;
-}
-
-// DualD (tangent) stage and finalize: value arrays in a.in_* / a.out_* /
-// a.un_* / a.n, tangent arrays in a.tan. Grid from stage_dual_grid_size().
-int launch_stage_dual(const StageArgs& a, int grid, void* stream, int lanes) {
-  k_stage<DualD><<<dim3(grid, lanes), NTHREADS, sizeof(StageSmemT<DualD>),
-                   (cudaStream_t)stream>>>(a);
-  return launched(stream);
-}
-
+// DualD forward-Euler finalize (the stage: hf_dual.cu). Grid from
+// stage_dual_grid_size().
 int launch_finalize_dual(const StageArgs& a, int grid, void* stream, int lanes) {
   k_finalize<DualD><<<dim3(grid, lanes), NTHREADS, 0, (cudaStream_t)stream>>>(a);
   return launched(stream);
