@@ -126,21 +126,23 @@ __global__ void __launch_bounds__(NTHREADS, 2) k_stage_adj(const StageArgs A, co
   const double dt = ctrl->dt;
   const int nr = A.nr, nc = A.nc;
   const double dx = A.dx, dy = A.dy;
-  const double dt_dx = dt / dx;
-  const double dt_dy = dt / dy;
   const double half_dx = 0.5 * dx, half_dy = 0.5 * dy;
   const double inv_dx = 1.0 / dx, inv_dy = 1.0 / dy;
   const int tid = threadIdx.x;
   const int ntiles = A.tiles_x * A.tiles_y;
-  if (tid == 0) S.extreme = 0;
+  if (tid == 0) {
+    S.extreme = 0;
+    stage_step_dt(A, S.dt);
+  }
   __syncthreads();
+  const double dt_dx = S.dt.over_dx, dt_dy = S.dt.over_dy;
 
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     const int tyi = tile / A.tiles_x;
     const int gi0 = tyi * TY, gj0 = (tile - tyi * A.tiles_x) * TX;
     const bool mod = (interior_tile(A, tile)
-                          ? stage_tile_faces<double, false, true>(A, S, gi0, gj0, dt)
-                          : stage_tile_faces<double>(A, S, gi0, gj0, dt)) == TILE_MODERATE;
+                          ? stage_tile_faces<double, false, true>(A, S, gi0, gj0)
+                          : stage_tile_faces<double>(A, S, gi0, gj0)) == TILE_MODERATE;
 
     // ---- A: per tile cell, epilogue / combination / update in reverse
     int src_lo = 0, src_hi = 0;

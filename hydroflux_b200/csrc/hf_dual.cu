@@ -26,7 +26,10 @@ __global__ void __launch_bounds__(NTHREADS, HF_MIN_BLOCKS == 1 ? 1 : 2)
   unsigned long long nonfin = 0;
   __shared__ __align__(16) unsigned char lane_raw[sizeof(StageArgs)];
   StageArgs& L = *reinterpret_cast<StageArgs*>(lane_raw);
-  if (threadIdx.x == 0) lane_args(A, blockIdx.y, L);
+  if (threadIdx.x == 0) {
+    lane_args(A, blockIdx.y, L);
+    stage_step_dt(A, S.dt);
+  }
   __syncthreads();
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     if (interior_tile(L, tile))

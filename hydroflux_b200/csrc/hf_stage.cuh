@@ -28,6 +28,12 @@ constexpr int FXW = TX + 3, FXH = TY + 2, FXN = FXW * FXH;  // x faces: rows [-1
 constexpr int FYW = TX + 2, FYH = TY + 3, FYN = FYW * FYH;  // y faces: faces [-1,TY+1], cols [-1,TX]
 constexpr int AW = TX + 2, AH = TY + 2, AN = AW * AH;       // alpha: rows [-1,TY], cols [-1,TX]
 
+// The step's dt and its ratios to the spacing (update.rs:930-931), divided once
+// per CTA (stage_step_dt) instead of by every thread for every tile.
+struct StepDt {
+  double t, over_dx, over_dy;
+};
+
 // The dry cells (h <= H_DRY, inside the grid) of a row of the tile and its
 // halo: bit c is column c - 4. The limiter, the faces and the update test
 // dryness about 22 times per cell; a test of bits takes none of the FP64 pipe
@@ -56,6 +62,7 @@ template <class T> struct StageSmemT {
   T fym[FYN], fynm[FYN], fynp[FYN], fyt[FYN];
   T a[AN];
   DryRow dry[R4H];
+  StepDt dt;
 };
 using StageSmem = StageSmemT<double>;
 
@@ -80,6 +87,7 @@ template <> struct StageSmemT<DualD> {
     DualD a[AN];
   };
   DryRow dry[R4H];
+  StepDt dt;
 };
 
 // The cells of the tile with its 4-cell halo by warps: rows of 32 columns,
@@ -673,7 +681,7 @@ __device__ __forceinline__ bool moderate_cell(double h, double z, double hu, dou
 }
 template <class T, bool PF = false, bool IN = false, bool DRY = false, bool HD = false>
 __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageSmemT<T>& S, int gi0,
-                                                 int gj0, double dt, double* hst = nullptr,
+                                                 int gj0, double* hst = nullptr,
                                                  int next = -1,
                                                  const StageArgs* next_args = nullptr) {
   constexpr bool SKIP = DRY && IN;
@@ -681,8 +689,6 @@ __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageS
   bool dry = true, mod = A.rx.moderate && A.ry.moderate;
   const int nr = A.nr, nc = A.nc;
   const double dx = A.dx, dy = A.dy;
-  const double dt_dx = dt / dx;  // update.rs:930-931
-  const double dt_dy = dt / dy;
   const double half_dx = 0.5 * dx, half_dy = 0.5 * dy;
   const int tid = threadIdx.x;
   const T Z = cst<T>(0.0);
@@ -992,6 +998,7 @@ __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageS
     }
 
     // ---- alpha mass rescaling factors: update.rs:953-982 (tile + 1-cell ring)
+    const double dt_dx = S.dt.over_dx, dt_dy = S.dt.over_dy;
     for (int k = tid; k < AN; k += NTHREADS) {
       const int r = k / AW;
       const int li = r - 1, lj = k - r * AW - 1;
@@ -1027,11 +1034,8 @@ __device__ __forceinline__ TileClass stage_tile(const StageArgs& A, StageSmemT<T
                                                 int next = -1,
                                                 const StageArgs* next_args = nullptr) {
   Ctrl* ctrl = A.ctrl;
-  const double dt = ctrl->dt;
   const int nr = A.nr, nc = A.nc;
   const double dx = A.dx, dy = A.dy;
-  const double dt_dx = dt / dx;  // update.rs:930-931
-  const double dt_dy = dt / dy;
   const int tid = threadIdx.x;
   const T Z = cst<T>(0.0);
   {
@@ -1039,7 +1043,7 @@ __device__ __forceinline__ TileClass stage_tile(const StageArgs& A, StageSmemT<T
     const int gi0 = tyi * TY, gj0 = (tile - tyi * A.tiles_x) * TX;
     // Dry interior tiles skip their slopes, faces and alpha (f64 forward stage).
     const TileClass cls = stage_tile_faces<T, PF, IN, std::is_same<T, double>::value, HD>(
-        A, S, gi0, gj0, dt, hst, next, next_args);
+        A, S, gi0, gj0, hst, next, next_args);
     const bool mod = cls == TILE_MODERATE;
     // A source term's division by the spacing (moderate tiles: unguarded).
     auto over = [mod](T a, const hfa::RecipD& r) -> T {
@@ -1050,6 +1054,7 @@ __device__ __forceinline__ TileClass stage_tile(const StageArgs& A, StageSmemT<T
     };
 
     // ---- FV update + bed source + floor: update.rs:1071-1210
+    const double dt = S.dt.t, dt_dx = S.dt.over_dx, dt_dy = S.dt.over_dy;
     int src_lo = 0, src_hi = 0;
     if (A.finalize && A.f.n_src > 0) {
       const int b = source_bucket(tile, A.tiles_x);
@@ -1194,6 +1199,14 @@ __device__ __forceinline__ void stage_tile_dry(const StageArgs& A, const double*
     A.out_hu[g] = nhu;
     A.out_hv[g] = nhv;
   }
+}
+
+// One thread, before the CTA's first tile of a grid and a barrier.
+__device__ __forceinline__ void stage_step_dt(const StageArgs& A, StepDt& d) {
+  const double dt = A.ctrl->dt;
+  d.t = dt;
+  d.over_dx = dt / A.dx;
+  d.over_dy = dt / A.dy;
 }
 
 // A tile whose 4-cell halo lies inside the grid reaches no side: it runs the

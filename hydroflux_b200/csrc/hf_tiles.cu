@@ -51,7 +51,10 @@ __global__ void __launch_bounds__(NTHREADS, HF_MIN_BLOCKS) k_stage_pf(const Stag
   const int ntiles = A.tiles_x * A.tiles_y;
   double sxm = 0.0, sym = 0.0;
   unsigned long long nonfin = 0;
-  if (threadIdx.x == 0) P.s.extreme = 0;
+  if (threadIdx.x == 0) {
+    P.s.extreme = 0;
+    stage_step_dt(A, P.s.dt);
+  }
   if ((int)blockIdx.x < ntiles) stage_prefetch(A, P.s, P.hst, blockIdx.x);
   int tile = blockIdx.x;
   while (tile < ntiles) {
@@ -199,7 +202,7 @@ __global__ void __launch_bounds__(NTHREADS, HF_MIN_BLOCKS)
   StagePfSmem& P = *reinterpret_cast<StagePfSmem*>(smem_raw);
   __shared__ __align__(16) unsigned char args_raw[sizeof(StageArgs)];
   StageArgs& A = *reinterpret_cast<StageArgs*>(args_raw);
-  __shared__ int claimed;
+  __shared__ int claimed, active;  // active: of the scenario in A
   const int total_tiles = *n_tiles;  // device-resident: a graph serves any set of scenarios
   int t = blockIdx.x;
   if (threadIdx.x == 0) P.s.extreme = 0;
@@ -227,12 +230,16 @@ __global__ void __launch_bounds__(NTHREADS, HF_MIN_BLOCKS)
       const unsigned long long* src = reinterpret_cast<const unsigned long long*>(&args[scn]);
       unsigned long long* dst = reinterpret_cast<unsigned long long*>(args_raw);
       for (int w = threadIdx.x; w < (int)(sizeof(StageArgs) / 8); w += NTHREADS) dst[w] = src[w];
+      if (threadIdx.x == NTHREADS - 1) {
+        active = args[scn].ctrl->active;
+        stage_step_dt(args[scn], P.s.dt);
+      }
       cur = scn;
     }
     if (counter && threadIdx.x == 0) claimed = atomicAdd(counter, 1);
     cp_async_wait_all();
     __syncthreads();  // this tile's inputs and A are in shared memory; the claim is visible
-    live = A.ctrl->active != 0;  // uniform over the CTA
+    live = active != 0;  // uniform over the CTA
     const int tn = counter ? claimed : t + (int)gridDim.x;
     const StageArgs* An = nullptr;
     if (tn < total_tiles) {
