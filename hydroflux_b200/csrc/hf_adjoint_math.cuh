@@ -29,7 +29,8 @@ HF_ADJ_HD double dmax0(double x) { return x > 0.0 ? 1.0 : (x < 0.0 ? 0.0 : 0.5);
 
 // Quotients and roots of forward values in the reverse faces. MOD (the face of
 // a moderate tile): the unguarded forms, whose values are the same, with one
-// reciprocal per divisor. A face divides by six values, thirteen times.
+// reciprocal per divisor. A face divides by six values, thirteen times
+// (gradient at 512^2, 48 steps: 20.8 -> 20.3 ms).
 template <bool MOD> HF_ADJ_HD double rev_recip(double b) {
   if (MOD && !hfa::low_word_ones(b)) return hfa::recip_rn(b);
   return 1.0 / b;
