@@ -433,20 +433,19 @@ void set_geom(hf_sim* s, int geom) {
 
 // Picks the stage kernel: the strip kernel where it is asked for and its TMA
 // descriptors can be made, else the tile kernel of the geometry asked for;
-// auto takes the tile kernel of the grid's geometry (geom_pick: on B200 the
+// auto takes the tile kernel of the grid's geometry (geom_for: on B200 the
 // tile kernel measured faster than the strip kernel on wet grids and as fast
 // on mostly dry ones). The strip kernel's grids keep the 32 x 8 geometry for
 // the CFL reduction and the forward-Euler finalize.
 int choose_stage_kernel(hf_sim* s, int kind) {
   const int64_t tx = tiles_along(s->nc, TX);
   const int geom = kind == HF_STAGE_TILE32 ? kGeomLarge
-                   : kind == HF_STAGE_AUTO ? geom_pick(s->nr, s->nc)
+                   : kind == HF_STAGE_AUTO ? geom_for(s->nr, s->nc)
                    : kind == HF_STAGE_TILE
                        ? small_geom(tx * tiles_along(s->nr, 8), tx * tiles_along(s->nr, 4))
                        : kGeomSmall;
   set_geom(s, geom);
-  const int as = kind == HF_STAGE_AUTO ? geom_for(s->nr, s->nc) : geom;
-  s->stage_kind = as == kGeomLarge ? HF_STAGE_TILE32 : HF_STAGE_TILE;
+  s->stage_kind = geom == kGeomLarge ? HF_STAGE_TILE32 : HF_STAGE_TILE;
   if (kind != HF_STAGE_STRIP) return HF_OK;
   int g = strip_grid_size(s->nr, s->nc, s->device);
   if (g == 0) {  // a small grid: one CTA per block at most
@@ -657,7 +656,7 @@ int hf_sim_create(const hf_mesh_desc* mesh, const double* h, const double* hu, c
   s->dx = mesh->dx;
   s->dy = mesh->dy;
   s->cfg = *cfg;
-  set_geom(s, geom_pick(s->nr, s->nc));
+  set_geom(s, geom_for(s->nr, s->nc));
   int rc = HF_OK;
   auto done = [&](int code) {
     if (code != HF_OK) destroy_sim(s);

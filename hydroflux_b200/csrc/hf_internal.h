@@ -15,8 +15,8 @@ namespace hf {
 // of cells, one cell per thread; its shared-memory halo is 4 cells (two-cell
 // dry buffer of the slope limiter + one neighbour slope + one neighbour
 // alpha). hf_tiles.cu is compiled once for each geometry, whose symbols sit in
-// its inline namespace; geom_pick() says which one a grid takes. Two carry the
-// grids that fill the GPU:
+// its inline namespace; geom_for() and geom_pick() say which one a grid takes.
+// Two carry the grids that fill the GPU:
 // - 32 x 8 (g8, kGeomSmall): 256 threads, 71 KB of shared memory, three CTAs
 //   (24 warps) per SM. Many tiles per grid, so small grids still spread over
 //   every SM. The DualD tangent, the adjoint, the strip kernel and the
@@ -297,15 +297,21 @@ const GeomOps& geom_ops_g8w();
 const GeomOps& geom_ops_g8m();
 const GeomOps& geom_ops_g4();
 const GeomOps& geom_ops(int geom);
-// The stage kernel kind a simulation reports for an nr x nc grid: kGeomLarge
-// once it has kLargeTilesMin tiles of 32 x 32, else kGeomSmall.
+// The geometry of a simulation of nr x nc cells whose stage kernel is left to
+// the library, on the current device: kGeomLarge from kLargeTilesMin tiles of
+// 32 x 32 on, else the small geometry that fills the SMs. The limit is part of
+// the interface (hf_sim_set_stage_kernel), and hf_sim_stage_kernel reports the
+// tiles that run: below about 2,300 tiles of 32 x 8 the waves of geom_pick would
+// sometimes take the small ones (us a step with small and large tiles, wet:
+// 320^2 35.0 / 38.7, 199 x 481 34.0 / 38.6, 400^2 50.0 / 63.5,
+// 450 x 500 69.2 / 65.9, 512^2 69.7 / 65.5, 600^2 85.2 / 91.4,
+// 640^2 99.6 / 92.0, 800^2 141.4 / 142.9, 1024^2 222.4 / 194.0).
 int geom_for(int64_t nr, int64_t nc);
-// The geometry that runs it on the current device. Tiles of 32 x 8 or 32 x 32
-// by the time of their waves (3 and 1 tiles per SM; a wave of a step takes
-// about 19 to 24 and 28.5 us; us a step with small and large tiles, wet:
-// 199 x 481 39.0 / 45.2, 400^2 60 / 74, 450 x 500 80 / 75, 512^2 78 / 77,
-// 700 x 500 95 / 102, 1024^2 242 / 214), and among the small ones
-// (small_geom) the CTA that fills the SMs.
+// The geometry of a free function's grid on the current device. Tiles of
+// 32 x 8 or 32 x 32 by the time of their waves (3 and 1 tiles per SM; a wave
+// of a step takes about 19 to 24 and 28.5 us), and among the small ones
+// (small_geom) the CTA that fills the SMs. Of the grids above it takes the
+// slower tiles at 640^2 alone.
 int geom_pick(int64_t nr, int64_t nc);
 // Whether n8 tiles of 32 x 8 take less time than n32 of 32 x 32 on the device.
 bool small_tiles_pay(int64_t n8, int64_t n32);

@@ -341,11 +341,6 @@ const GeomOps& geom_ops(int geom) {
   }
 }
 
-int geom_for(int64_t nr, int64_t nc) {
-  const int64_t t = (int64_t)tiles_along(nc, TX) * tiles_along(nr, kGeomTileH[kGeomLarge]);
-  return t >= kLargeTilesMin ? kGeomLarge : kGeomSmall;
-}
-
 int64_t sm_count() {
   int dev = 0, sms = 0;
   if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -365,6 +360,12 @@ int small_geom(int64_t n8, int64_t n4) {
   const int64_t sms = sm_count();
   if (n4 > 0 && n4 <= sms) return kGeomLow;
   return n8 <= sms ? kGeomWide : n8 <= 2 * sms ? kGeomMid : kGeomSmall;
+}
+int geom_for(int64_t nr, int64_t nc) {
+  const int64_t tx = tiles_along(nc, TX);
+  return tx * tiles_along(nr, 32) >= kLargeTilesMin
+             ? kGeomLarge
+             : small_geom(tx * tiles_along(nr, 8), tx * tiles_along(nr, 4));
 }
 int geom_pick(int64_t nr, int64_t nc) {
   const int64_t tx = tiles_along(nc, TX), n8 = tx * tiles_along(nr, 8);

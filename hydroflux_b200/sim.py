@@ -350,8 +350,8 @@ class Simulation:
     def set_stage_kernel(self, kind: str) -> None:
         """'tile' (32 x 8 tiles, or 32 x 4 on small grids), 'tile32' (32 x 32
         tiles), 'strip' or 'auto' (hf_sim_set_stage_kernel): which kernel runs
-        the stages; auto takes the tiles that suit the grid and the device and
-        reports 'tile32' from 100 such tiles on."""
+        the stages; auto takes tile32 on grids of at least 100 tiles of 32 x 32,
+        else tile. Results are bit-identical."""
         raise_for(lib().hf_sim_set_stage_kernel(self._h, self.STAGE_KERNELS[kind]))
 
     def stage_kernel(self) -> str:

@@ -173,9 +173,8 @@ int hf_sim_set_boundaries(hf_sim* sim, const hf_boundaries* bcs);
  * HF_STAGE_STRIP walks 32-column strips in 7-row blocks and carries the halo
  * rows from block to block (fewer faces and slopes per cell, TMA row
  * fetches; needs an even column count). HF_STAGE_AUTO (the default at
- * creation) takes the tiles that take fewer and shorter waves on the device;
- * hf_sim_stage_kernel reports the kernel asked for, and for HF_STAGE_AUTO
- * HF_STAGE_TILE32 from 100 tiles of 32 x 32 on and HF_STAGE_TILE below.
+ * creation) takes HF_STAGE_TILE32 for grids of at least 100 tiles of 32 x 32
+ * and HF_STAGE_TILE below; hf_sim_stage_kernel reports the kernel in use.
  * Results are bit-identical; this is a tuning and diagnostic knob. Forcing
  * HF_STAGE_STRIP where it cannot run returns HF_ERR_UNSUPPORTED (the auto
  * choice stays selected). */
