@@ -438,12 +438,9 @@ void set_geom(hf_sim* s, int geom) {
 // on mostly dry ones). The strip kernel's grids keep the 32 x 8 geometry for
 // the CFL reduction and the forward-Euler finalize.
 int choose_stage_kernel(hf_sim* s, int kind) {
-  const int64_t tx = tiles_along(s->nc, TX);
-  const int geom = kind == HF_STAGE_TILE32 ? kGeomLarge
+  const int geom = kind == HF_STAGE_TILE32   ? kGeomLarge
                    : kind == HF_STAGE_AUTO ? geom_for(s->nr, s->nc)
-                   : kind == HF_STAGE_TILE
-                       ? small_geom(tx * tiles_along(s->nr, 8), tx * tiles_along(s->nr, 4))
-                       : kGeomSmall;
+                                           : kGeomSmall;
   set_geom(s, geom);
   s->stage_kind = geom == kGeomLarge ? HF_STAGE_TILE32 : HF_STAGE_TILE;
   if (kind != HF_STAGE_STRIP) return HF_OK;

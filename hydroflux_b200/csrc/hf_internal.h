@@ -28,13 +28,15 @@ namespace hf {
 //   takes 1.60 ms against 1.79 ms.
 // Grids that leave SMs idle are bound by the latency of one tile: its five
 // phases take about three passes of 256 threads each. They run on CTAs with
-// more threads per tile (us a step, wet with walls, 256 threads -> the other):
+// more threads per tile (us a step, wet with walls, 256 threads -> the other;
+// the figures that speak for the limits are from before the dry bits, when
+// every step took about 4 us more):
 // - 32 x 8, 768 threads (g8w, kGeomWide): one pass per phase, one CTA per SM;
-//   160 x 200 31.1 -> 26.2, but 256^2 (two tiles for some SMs) 35.3 -> 39.0.
+//   160 x 200 25.7 -> 22.1, but 256^2 (two tiles for some SMs) 35.3 -> 39.0.
 // - 32 x 8, 384 threads (g8m, kGeomMid): two passes, two CTAs per SM; 256^2
-//   35.3 -> 32.1, but 199 x 481 (400 tiles) 39.8 -> 44.7.
+//   29.7 -> 26.4, but 199 x 481 (400 tiles) 39.8 -> 44.7.
 // - 32 x 4, 512 threads (g4, kGeomLow): half the work per SM again; 48 x 64
-//   24.9 (g8w) -> 22.8.
+//   25.7 -> 19.3.
 // All compute every cell with the same operations: results are identical.
 constexpr int TX = 32;
 constexpr int kGeomSmall = 0, kGeomLarge = 1, kGeomWide = 2, kGeomMid = 3, kGeomLow = 4;

@@ -348,10 +348,11 @@ class Simulation:
     STAGE_KERNELS = {"auto": 0, "tile": 1, "strip": 2, "tile32": 3}
 
     def set_stage_kernel(self, kind: str) -> None:
-        """'tile' (32 x 8 tiles, or 32 x 4 on small grids), 'tile32' (32 x 32
-        tiles), 'strip' or 'auto' (hf_sim_set_stage_kernel): which kernel runs
-        the stages; auto takes tile32 on grids of at least 100 tiles of 32 x 32,
-        else tile. Results are bit-identical."""
+        """'tile' (32 x 8 tiles), 'tile32' (32 x 32 tiles), 'strip' or 'auto'
+        (hf_sim_set_stage_kernel): which kernel runs the stages; auto takes
+        tile32 on grids of at least 100 tiles of 32 x 32, else tile, on the
+        smallest grids with more threads per tile or tiles of 32 x 4. Results
+        are bit-identical."""
         raise_for(lib().hf_sim_set_stage_kernel(self._h, self.STAGE_KERNELS[kind]))
 
     def stage_kernel(self) -> str:

@@ -166,15 +166,17 @@ int hf_sim_set_state_aos(hf_sim* sim, const double* hhuhv);
 int hf_sim_set_boundaries(hf_sim* sim, const hf_boundaries* bcs);
 /* Which kernel runs the stages of a simulation; no counterpart in the
  * reference (its passes are fixed). HF_STAGE_TILE computes every 32 x 8
- * tile with its halo (three 256-thread CTAs per SM; on grids that leave SMs
- * idle fewer CTAs of more threads, down to 32 x 4 tiles); HF_STAGE_TILE32
- * every 32 x 32 tile (one 1024-thread CTA per SM: a smaller halo share, more
- * warps per SM; faster once a grid has enough tiles to fill the GPU);
+ * tile with its halo (three 256-thread CTAs per SM); HF_STAGE_TILE32 every
+ * 32 x 32 tile (one 1024-thread CTA per SM: a smaller halo share, more warps
+ * per SM; faster once a grid has enough tiles to fill the GPU);
  * HF_STAGE_STRIP walks 32-column strips in 7-row blocks and carries the halo
  * rows from block to block (fewer faces and slopes per cell, TMA row
  * fetches; needs an even column count). HF_STAGE_AUTO (the default at
  * creation) takes HF_STAGE_TILE32 for grids of at least 100 tiles of 32 x 32
- * and HF_STAGE_TILE below; hf_sim_stage_kernel reports the kernel in use.
+ * and HF_STAGE_TILE below, there with fewer CTAs of more threads, down to
+ * 32 x 4 tiles, on grids that leave SMs idle (at most two tiles of 32 x 8 per
+ * SM); hf_sim_stage_kernel reports the kernel in use, as HF_STAGE_TILE for
+ * each of these small tiles.
  * Results are bit-identical; this is a tuning and diagnostic knob. Forcing
  * HF_STAGE_STRIP where it cannot run returns HF_ERR_UNSUPPORTED (the auto
  * choice stays selected). */

@@ -57,3 +57,14 @@ def test_reported_kernel_is_the_launched_one():
     for case, (kind, names) in zip(cases, launched(cases)):
         assert len(names) == 1, (case, names)
         assert (kind == "tile32") == (names == ["g32"]), (case, kind, names)
+
+
+def test_forced_kernel_is_the_launched_one():
+    """'tile' is the 32 x 8 tile by 256 threads and 'tile32' the 32 x 32 one on
+    every grid, those too where auto takes other CTAs: up to 148 tiles of 32 x 4,
+    up to 148 and 296 of 32 x 8, and more."""
+    cases = [(kind, *shape) for shape in [(1, 1), (48, 64), (160, 200), (256, 256), (400, 400)]
+             for kind in ("tile", "tile32")]
+    for case, (kind, names) in zip(cases, launched(cases)):
+        assert kind == case[0]
+        assert names == ["g8" if kind == "tile" else "g32"], (case, names)
