@@ -151,6 +151,15 @@ def measured_peaks():
 KERNEL_NAMES = {"tile": "k_stage_pf/32x8", "tile32": "k_stage_pf/32x32", "strip": "k_stage_strip"}
 
 
+def kernel_name(kind, asked, n, sms):
+    """The name of the kernel that runs an n x n grid, for the reported kind and
+    the one asked for. The small tiles that 'auto' takes on at most two tiles of
+    32 x 8 per SM have other CTAs than the profiled ones: no figures."""
+    if kind == "tile" and asked == "auto" and -(-n // 8) * -(-n // 32) <= 2 * sms:
+        return "k_stage_pf/small"
+    return KERNEL_NAMES[kind]
+
+
 def profiled_figure(kernel, key):
     """A per-cell figure of a stage kernel from the committed ncu summary
     (lines `<kernel>.<key>: value`)."""
@@ -279,7 +288,8 @@ def run_ours(a, d: Dist):
     bytes_per_launch = ALG_BYTES_PER_CELL_UPDATE / STAGE_LAUNCHES_PER_STEP * cells
     achieved_gbs = bytes_per_launch / avg_stage_s / 1e9
     peak, peak_kind = measured_peaks()
-    kernel = KERNEL_NAMES[sm.stage_kernel()]
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    kernel = kernel_name(sm.stage_kernel(), a.stage_kernel, a.n, sms)
     traffic_per_cell = profiled_traffic(kernel)
     sm.close()
 
@@ -438,7 +448,8 @@ def run_regimes(a, d: Dist):
                 e1.record(stream)
             torch.cuda.synchronize(dev)
             ms = d.max(e0.elapsed_time(e1))
-            kernel = sm.stage_kernel()
+            sms = torch.cuda.get_device_properties(dev).multi_processor_count
+            kernel = kernel_name(sm.stage_kernel(), "auto", a.n, sms)
             state = sm.states()
             t0 = sm.time()
         cpu = None
@@ -455,7 +466,7 @@ def run_regimes(a, d: Dist):
                    "sample": "1 step of the same state, CPU oracle, 1 thread"}
         out[kind] = {"value": d.world * scn.n_cells * a.steps / (ms / 1e3), "unit": UNIT,
                      "ms_per_step": ms / a.steps, "wet_fraction": round(wet, 4),
-                     "stage_kernel": KERNEL_NAMES[kernel],
+                     "stage_kernel": kernel,
                      "cpu_baseline": cpu}
     clk = clocks.stop()
     line = {"metric": "cell-updates/s (mostly dry)", "value": out["mostly_dry"]["value"],
