@@ -729,6 +729,7 @@ __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageS
     if (!mod) S.extreme = 1;
     if constexpr (SKIP) {
       if (__syncthreads_and(dry)) {
+        if (tid == 0) S.extreme = 0;  // not read; the update ends with a barrier
         if constexpr (!HD) {
           if (next >= 0) stage_prefetch(next_args ? *next_args : A, S, hst, next);
         }
@@ -785,7 +786,10 @@ __device__ __forceinline__ TileClass stage_tile_faces(const StageArgs& A, StageS
       if (!mod) S.extreme = 1;
     }
     if constexpr (SKIP) {
-      if (__syncthreads_and(dry)) return TILE_DRY;
+      if (__syncthreads_and(dry)) {
+        if (tid == 0) S.extreme = 0;
+        return TILE_DRY;
+      }
     } else {
       __syncthreads();
     }
