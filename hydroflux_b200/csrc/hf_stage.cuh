@@ -252,10 +252,13 @@ struct StagePfSmem {
   alignas(16) double hst[R4N];
 };
 // Depth buffers of a run of dry tiles (stage_dry_run), over the slopes, faces
-// and alpha that such tiles do not use.
+// and alpha that such tiles do not use, but below the dry bits and the step's
+// dt, which the tiles after the run read.
 constexpr int DRY_RING = 4;
-static_assert(sizeof(StageSmem) - offsetof(StageSmem, sxe) >= (DRY_RING * R4N + 1) * sizeof(double),
-              "the ring fits over the slopes and faces");
+static_assert(offsetof(StageSmem, dry) - offsetof(StageSmem, sxe) >=
+                      (DRY_RING * R4N + 1) * sizeof(double) &&
+                  offsetof(StageSmem, dt) > offsetof(StageSmem, dry),
+              "the ring fits over the slopes, faces and alpha");
 static_assert(R3W % 2 == 0 && R4W % 2 == 0 && TX % 2 == 0, "column pairs");
 static_assert(offsetof(StageSmem, h) % 16 == 0 && offsetof(StageSmem, eta) % 16 == 8 &&
                   offsetof(StageSmem, u) % 16 == 8 && offsetof(StageSmem, v) % 16 == 8 &&
