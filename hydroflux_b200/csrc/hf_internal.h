@@ -57,6 +57,9 @@ constexpr int kSoloTilesMin = 512;
 // The build of the 32 x 8 geometry also carries the kernels that exist in
 // one geometry only (strip, DualD, adjoint) and the host code.
 #define HF_GEOM_PRIMARY (HF_GEOM_INDEX == 0)
+// Ensembles and servers take tiles of 8 or 32 rows (hf_batch.cu, hf_serve.cu):
+// the 32 x 4 geometry has no batched kernels.
+#define HF_GEOM_BATCHED (HF_TILE_Y >= 8)
 #define HF_CAT2(a, b) a##b
 #define HF_CAT(a, b) HF_CAT2(a, b)
 #define HF_GEOM_OPS HF_CAT(geom_ops_, HF_GEOM)
@@ -288,6 +291,7 @@ struct GeomOps {
   int (*stage)(const StageArgs& a, int grid, void* stream);
   int (*finalize)(const StageArgs& a, int grid, void* stream);
   int (*cfl)(const StageArgs& a, int with_ghosts, int grid, void* stream);
+  // Null where the geometry has no batched kernels (HF_GEOM_BATCHED).
   int (*stage_batch)(const StageArgs* args, const int* tile_scn, const int* n_tiles, int grid,
                      void* stream, const int* tile_local, int* counter);
   int (*cfl_batch)(const StageArgs* args, const int* tile_scn, int first_tile, int last_tile,

@@ -1042,7 +1042,6 @@ __device__ __forceinline__ TileClass stage_tile(const StageArgs& A, StageSmemT<T
                                                 const StageArgs* next_args = nullptr) {
   Ctrl* ctrl = A.ctrl;
   const int nr = A.nr, nc = A.nc;
-  const double dx = A.dx, dy = A.dy;
   const int tid = threadIdx.x;
   const T Z = cst<T>(0.0);
   {

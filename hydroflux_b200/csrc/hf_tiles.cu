@@ -171,6 +171,7 @@ __global__ void __launch_bounds__(NTHREADS, HF_MIN_BLOCKS)
 }
 #endif  // HF_GEOM_PRIMARY
 
+#if HF_GEOM_BATCHED
 // One stage of every grid of an ensemble in one launch: the persistent grid
 // walks the concatenated tile list of all scenarios; tile t belongs to
 // scenario tile_scn[t], whose arguments (own sizes, dt, forcings, control
@@ -262,6 +263,7 @@ __global__ void __launch_bounds__(NTHREADS, HF_MIN_BLOCKS)
   }
   if (live && A.finalize) block_reduce_speeds(sxm, sym, nonfin, A.ctrl);
 }
+#endif  // HF_GEOM_BATCHED
 
 // Epilogue of a forward-Euler step: friction, forcings and the CFL
 // reduction of the stage result (in_*) into the state (out_*).
@@ -347,6 +349,7 @@ __global__ void __launch_bounds__(NTHREADS) k_cfl(const StageArgs A, int with_gh
   if (blockIdx.x == 0 && threadIdx.x == 0) ctrl->cfl_valid = 1;
 }
 
+#if HF_GEOM_BATCHED
 // Ensemble CFL reduction (with ghosts), reduced per tile into its scenario.
 __global__ void __launch_bounds__(NTHREADS)
     k_cfl_batch(const StageArgs* __restrict__ args, const int* __restrict__ tile_scn,
@@ -370,6 +373,7 @@ __global__ void __launch_bounds__(NTHREADS)
     block_reduce_speeds(sxm, sym, nonfin, A.ctrl);
   }
 }
+#endif  // HF_GEOM_BATCHED
 
 // ------------------------------------------------------------- launchers
 size_t stage_smem_bytes() { return sizeof(StageSmem); }
@@ -383,8 +387,10 @@ int stage_grid_size(int tiles, int device) {
     DevGuard dg(device);
     cudaFuncSetAttribute(k_stage_pf, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(StagePfSmem));
+#if HF_GEOM_BATCHED
     cudaFuncSetAttribute(k_stage_batch, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)sizeof(StagePfSmem));
+#endif
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_stage_pf, NTHREADS,
                                                   sizeof(StagePfSmem));
     if (per_sm < 1) per_sm = 1;
@@ -487,6 +493,7 @@ int launch_finalize(const StageArgs& a, int grid, void* stream) {
   return launched(stream);
 }
 
+#if HF_GEOM_BATCHED
 int launch_stage_batch(const StageArgs* args, const int* tile_scn, const int* n_tiles, int grid,
                        void* stream, const int* tile_local, int* counter) {
   k_stage_batch<<<grid, NTHREADS, sizeof(StagePfSmem), (cudaStream_t)stream>>>(
@@ -500,6 +507,7 @@ int launch_cfl_batch(const StageArgs* args, const int* tile_scn, int first_tile,
   k_cfl_batch<<<grid, NTHREADS, 0, (cudaStream_t)stream>>>(args, tile_scn, first_tile, last_tile);
   return launched(stream);
 }
+#endif  // HF_GEOM_BATCHED
 
 int launch_cfl(const StageArgs& a, int with_ghosts, int grid, void* stream) {
   k_cfl<<<grid, NTHREADS, 0, (cudaStream_t)stream>>>(a, with_ghosts);
@@ -511,7 +519,13 @@ int launch_cfl(const StageArgs& a, int with_ghosts, int grid, void* stream) {
 // The geometry's entry points, for geom_ops().
 const GeomOps& HF_GEOM_OPS() {
   static const GeomOps ops = {TY, NTHREADS, &stage_grid_size, &launch_stage, &launch_finalize,
-                              &launch_cfl, &launch_stage_batch, &launch_cfl_batch};
+                              &launch_cfl,
+#if HF_GEOM_BATCHED
+                              &launch_stage_batch, &launch_cfl_batch
+#else
+                              nullptr, nullptr
+#endif
+  };
   return ops;
 }
 
