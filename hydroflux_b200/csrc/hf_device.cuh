@@ -198,10 +198,12 @@ static __device__ __noinline__ FaceFlux wb_face_general(double hL, double qnL, d
 //   on the high word: a value within 2^-20 above one counts as a failed
 //   condition. sl and sr, sums with a root > 0, are never -0 or below 2^-253;
 //   s_star may be -0, the one value with the high word 0x80000000, which is
-//   >= 0. (256^2 dam break, 23 steps: 579 -> 552 us.)
+//   >= 0. (256^2 dam break, intervals of 0.4 s: 579 -> 552 us.)
 //
-// Per face this is about 150 FP64 operations, the floor of a stage that is
-// bound by the FP64 pipe (two cycles per warp instruction and scheduler).
+// Per face this is about 150 FP64 operations, two cycles of a scheduler per
+// warp each. They are not the bound by themselves: on the 2048^2 valley the FP64
+// pipe is 36% busy and the issue slots 57%, with barriers and dependent
+// operations in the rest (profiles/stage_kernel32_valley2048.md).
 __device__ __forceinline__ constexpr int high_word(double x) {  // of a positive constant
   return (int)(__builtin_bit_cast(unsigned long long, x) >> 32);
 }
